@@ -637,6 +637,8 @@ mg_status mg_sweep_options(mg_ctx *ctx, const mg_sweep_opts *opts) {
     ctx->mws.giant_class = gc;
     ctx->mws.coarsen_combine = comb;
     ctx->mws.first_sweep_kernels = !(opts && opts->table_first_sweep);
+    ctx->mws.forced_policy = opts && (fill != MG_FILL_AUTO || opts->giant_class || opts->light_streams ||
+                                      opts->table_first_sweep);
     ctx->mws.light_streams =
         opts && opts->light_streams ? opts->light_streams : MoveWorkspace::kDefaultLightStreams;
     return MG_OK;

@@ -8,6 +8,8 @@
 #include "common.cuh"
 #include "primitives.cuh"
 
+struct mg_ctx;
+
 namespace mg {
 
 // Read-only view of a CSR level on the device.  Offsets are 32-bit (every
@@ -181,6 +183,11 @@ struct MoveWorkspace {
     DBuf<SweepAcc> acc;
     DBuf<SweepAcc> tune_acc;       // sums of the autotuner's timing runs (discarded)
     TuneTable tune;
+    // the policy is not the default one (mg_sweep_options): every sweep takes
+    // the kernels it names, also on levels that the resident kernel would run
+    bool forced_policy = false;
+    DBuf<unsigned char> resident;  // resident level kernel: state, sums, counters, barrier
+    void *h_resident = nullptr;    // pinned image of them
     PrimWorkspace prim;
     // stream 0: heavy tiers; streams 1..light_streams: the light classes and
     // the class-13 tier, so that one class's tail overlaps the others (one by
@@ -296,6 +303,24 @@ void sigma_update(const uint32_t *P, const uint32_t *N, const double *k, double 
 void level_init(const GraphView &g, double *k, double *sigma, uint32_t *C, cudaStream_t s);
 // Q = sum_in/mass - s2/mass^2 from host-side copy of the accumulators
 double modularity_from_acc(const SweepAcc &a, double mass, int integral);
+
+// Small levels: all iterations of a level in one kernel (resident.cuh).  The
+// line lies where the two paths meet: one CTA per SM keeps fewer warps in
+// flight than the class kernels, which counts once a sweep takes longer than
+// their launches.  SBM runs, local move only, resident / class kernels: 1.0 M
+// entries 2.9 / 6.0 ms, 4.0 M 6.9 / 9.4, 10 M 15.7 / 16.7, 24 M 38.7 / 31.5;
+// Chung-Lu, 15 M entries: 16.8 / 19.1 ms.
+constexpr uint64_t kResidentMaxEntries = 12u << 20;
+struct ResidentResult {
+    int base = 0;                            // buffer holding the accepted assignment
+    std::vector<double> Q;                   // per sweep: Q of its input assignment
+    std::vector<unsigned long long> distinct;  // per sweep: candidate pairs
+};
+bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws);
+// Iterates the prepared level (k, sigma, C[0] set by level_init, classes by
+// move_prepare_level) to its end.
+void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,
+                  ResidentResult &out, cudaStream_t s);
 
 // Coarsening.  out_off/out_col/out_w are resized as needed.
 struct CoarsenWorkspace {

@@ -154,6 +154,7 @@ MoveWorkspace::~MoveWorkspace() {
         if (e) cudaEventDestroy(e);
     for (auto &e : ev_tune)
         if (e) cudaEventDestroy(e);
+    if (h_resident) cudaFreeHost(h_resident);
 }
 
 void MoveWorkspace::init_streams() {

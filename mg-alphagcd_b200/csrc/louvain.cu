@@ -135,73 +135,99 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         Timer tp(ctx->ev[0], ctx->ev[1], s);
         level_init(cur, k, sigma, C[0], s);
         move_prepare_level(cur, mlv, ctx->mws, s);
-        int base = 0, pend = 1;
-        // first sweep: P = identity (base), proposes C[1]; yields Q0
-        sp.up = 1;
-        sp.agg = 0;
-        sp.split = sweep_split(ctx->mws, 0);
-        sp.first = ctx->mws.first_sweep_kernels && cur.sorted_rows;
-        // shapes of the light classes from the tuning table; classes missing
-        // from it are timed on the level's second sweep, which is more like
-        // the rest of the level than the first (every community one vertex)
-        move_tune(cur, mlv, ctx->mws, sp, C[base], C[pend], k, sigma, s, false);
-        sweep_reset_acc(ctx->mws, s);
-        sigma_sumsq(sigma, n, integral, ctx->mws, s);
-        MG_CUDA(cudaEventRecord(ctx->ev[4], s));
-        move_sweep(cur, mlv, ctx->mws, sp, C[base], C[pend], k, sigma, s);
-        MG_CUDA(cudaEventRecord(ctx->ev[5], s));
-        MG_CUDA(cudaMemcpyAsync(&hacc, ctx->mws.acc.get(), sizeof(SweepAcc), cudaMemcpyDeviceToHost, s));
-        double lm = tp.stop_sync();
-        phase_lm += lm;
-        account_sweep(ctx, cur, hacc, S);
-        S.sweeps++;
-        S.edges_swept += cur.nnz;
-        S.distinct_pairs += hacc.distinct;
-        if (phase == 0) {
-            S.phase0_edges_swept += cur.nnz;
-        }
-        double curQ = modularity_from_acc(hacc, mass, integral);
-        res.trace.insert(res.trace.end(), {(double)phase, 0.0, curQ, 0.0});
-        if (verbose) printf("| %-10d | %-10f | %-10f | %-10f | %-10f |\n", 0, curQ, 0., 0., 0.);
-        sigma_update(C[base], C[pend], k, sigma, n, ctx->mws, s);
-        int loop = 0;
-        while (true) {
-            sp.up = !sp.up;
-            // combine equal communities in the warp once they repeat: fewer
-            // than half of the last sweep's edges were distinct candidates
-            sp.first = 0;
-            sp.agg = 2 * hacc.distinct < cur.nnz;
-            sp.split = sweep_split(ctx->mws, sp.agg);
-            const int next = 3 - base - pend;
-            // autotuner: its timing runs write the proposal this sweep writes
-            if (loop == 0) move_tune(cur, mlv, ctx->mws, sp, C[pend], C[next], k, sigma, s, true);
-            Timer ti(ctx->ev[0], ctx->ev[1], s);
+        int base = 0, loop = 0;
+        double curQ = 0;
+        unsigned long long last_distinct = 0;
+        auto account = [&](unsigned long long distinct) {
+            S.sweeps++;
+            S.edges_swept += cur.nnz;
+            S.distinct_pairs += distinct;
+            if (phase == 0) S.phase0_edges_swept += cur.nnz;
+            last_distinct = distinct;
+        };
+        // (the printed table has a time per iteration: verbose runs take the
+        // iteration-by-iteration path)
+        if (!verbose && resident_level(cur, mlv, ctx->mws)) {
+            ResidentResult R;
+            MG_CUDA(cudaEventRecord(ctx->ev[4], s));
+            resident_run(ctx, cur, mlv, sp, thr, R, s);
+            MG_CUDA(cudaEventRecord(ctx->ev[5], s));
+            phase_lm += tp.stop_sync();
+            float ms = 0;
+            MG_CUDA(cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]));
+            S.seconds_sweep_kernels += ms * 1e-3;
+            for (size_t i = 0; i < R.Q.size(); i++) {
+                account(R.distinct[i]);
+                S.sweep_bytes += 12.0 * (double)cur.nnz + 24.0 * (double)n + 8.0 * (double)R.distinct[i];
+                // every sweep but the last was accepted
+                const bool last = i + 1 == R.Q.size();
+                if (i == 0) res.trace.insert(res.trace.end(), {(double)phase, 0.0, R.Q[0], 0.0});
+                else if (!last) res.trace.insert(res.trace.end(), {(double)phase, (double)i, R.Q[i], R.Q[i] - curQ});
+                else res.trace.insert(res.trace.end(), {(double)phase, (double)i, curQ, 0.0});
+                if (!last) curQ = R.Q[i];
+            }
+            loop = (int)R.Q.size() - 1;
+            base = R.base;
+        } else {
+            int pend = 1;
+            // first sweep: P = identity (base), proposes C[1]; yields Q0
+            sp.up = 1;
+            sp.agg = 0;
+            sp.split = sweep_split(ctx->mws, 0);
+            sp.first = ctx->mws.first_sweep_kernels && cur.sorted_rows;
+            // shapes of the light classes from the tuning table; classes missing
+            // from it are timed on the level's second sweep, which is more like
+            // the rest of the level than the first (every community one vertex)
+            move_tune(cur, mlv, ctx->mws, sp, C[base], C[pend], k, sigma, s, false);
             sweep_reset_acc(ctx->mws, s);
             sigma_sumsq(sigma, n, integral, ctx->mws, s);
             MG_CUDA(cudaEventRecord(ctx->ev[4], s));
-            move_sweep(cur, mlv, ctx->mws, sp, C[pend], C[next], k, sigma, s);
+            move_sweep(cur, mlv, ctx->mws, sp, C[base], C[pend], k, sigma, s);
             MG_CUDA(cudaEventRecord(ctx->ev[5], s));
             MG_CUDA(cudaMemcpyAsync(&hacc, ctx->mws.acc.get(), sizeof(SweepAcc), cudaMemcpyDeviceToHost, s));
-            double dt = ti.stop_sync();
-            phase_lm += dt;
+            double lm = tp.stop_sync();
+            phase_lm += lm;
             account_sweep(ctx, cur, hacc, S);
-            S.sweeps++;
-            S.edges_swept += cur.nnz;
-            S.distinct_pairs += hacc.distinct;
-            if (phase == 0) S.phase0_edges_swept += cur.nnz;
-            loop++;
-            const double Qp = modularity_from_acc(hacc, mass, integral);
-            if ((Qp - curQ) > thr) {
-                res.trace.insert(res.trace.end(), {(double)phase, (double)loop, Qp, Qp - curQ});
-                if (verbose) printf("| %-10d | %-10f | %-10f | %-10f | %-10f |\n", loop, Qp, Qp - curQ, dt, dt * 1e3);
-                curQ = Qp;
-                sigma_update(C[pend], C[next], k, sigma, n, ctx->mws, s);
-                base = pend;
-                pend = next;
-            } else {
-                res.trace.insert(res.trace.end(), {(double)phase, (double)loop, curQ, 0.0});
-                if (verbose) printf("| %-10d | %-10f | %-10f | %-10f | %-10f |\n", loop, curQ, 0., dt, dt * 1e3);
-                break;
+            account(hacc.distinct);
+            curQ = modularity_from_acc(hacc, mass, integral);
+            res.trace.insert(res.trace.end(), {(double)phase, 0.0, curQ, 0.0});
+            if (verbose) printf("| %-10d | %-10f | %-10f | %-10f | %-10f |\n", 0, curQ, 0., 0., 0.);
+            sigma_update(C[base], C[pend], k, sigma, n, ctx->mws, s);
+            while (true) {
+                sp.up = !sp.up;
+                // combine equal communities in the warp once they repeat: fewer
+                // than half of the last sweep's edges were distinct candidates
+                sp.first = 0;
+                sp.agg = 2 * hacc.distinct < cur.nnz;
+                sp.split = sweep_split(ctx->mws, sp.agg);
+                const int next = 3 - base - pend;
+                // autotuner: its timing runs write the proposal this sweep writes
+                if (loop == 0) move_tune(cur, mlv, ctx->mws, sp, C[pend], C[next], k, sigma, s, true);
+                Timer ti(ctx->ev[0], ctx->ev[1], s);
+                sweep_reset_acc(ctx->mws, s);
+                sigma_sumsq(sigma, n, integral, ctx->mws, s);
+                MG_CUDA(cudaEventRecord(ctx->ev[4], s));
+                move_sweep(cur, mlv, ctx->mws, sp, C[pend], C[next], k, sigma, s);
+                MG_CUDA(cudaEventRecord(ctx->ev[5], s));
+                MG_CUDA(cudaMemcpyAsync(&hacc, ctx->mws.acc.get(), sizeof(SweepAcc), cudaMemcpyDeviceToHost, s));
+                double dt = ti.stop_sync();
+                phase_lm += dt;
+                account_sweep(ctx, cur, hacc, S);
+                account(hacc.distinct);
+                loop++;
+                const double Qp = modularity_from_acc(hacc, mass, integral);
+                if ((Qp - curQ) > thr) {
+                    res.trace.insert(res.trace.end(), {(double)phase, (double)loop, Qp, Qp - curQ});
+                    if (verbose) printf("| %-10d | %-10f | %-10f | %-10f | %-10f |\n", loop, Qp, Qp - curQ, dt, dt * 1e3);
+                    curQ = Qp;
+                    sigma_update(C[pend], C[next], k, sigma, n, ctx->mws, s);
+                    base = pend;
+                    pend = next;
+                } else {
+                    res.trace.insert(res.trace.end(), {(double)phase, (double)loop, curQ, 0.0});
+                    if (verbose) printf("| %-10d | %-10f | %-10f | %-10f | %-10f |\n", loop, curQ, 0., dt, dt * 1e3);
+                    break;
+                }
             }
         }
         S.iterations += loop;  // the reference's loop count (moves evaluated)
@@ -228,7 +254,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
             break;
         }
         coarsen_level(cur, Cd, nn, integral, ctx->lv[lvl_out], ctx->cws, s, nullptr,
-                      coarsen_combine(ctx->mws, hacc.distinct, cur.nnz));
+                      coarsen_combine(ctx->mws, last_distinct, cur.nnz));
         double ct = tc.stop_sync();
         S.seconds_coarsen += ct;
         if (verbose) printf("Coarsen graph execution time: %f s, %f ms\n", ct, ct * 1e3);

@@ -1,0 +1,12 @@
+// resident_f64.cu -- the resident level kernel for weight kind WK_F64.
+#include "resident.cuh"
+
+namespace mg {
+namespace lmr {
+
+void launch_resident_f64(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
+    launch_resident_kind<WK_F64>(A, prec, ver, grid, s);
+}
+
+}  // namespace lmr
+}  // namespace mg

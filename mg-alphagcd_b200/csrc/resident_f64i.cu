@@ -1,0 +1,12 @@
+// resident_f64i.cu -- the resident level kernel for weight kind WK_F64I.
+#include "resident.cuh"
+
+namespace mg {
+namespace lmr {
+
+void launch_resident_f64i(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
+    launch_resident_kind<WK_F64I>(A, prec, ver, grid, s);
+}
+
+}  // namespace lmr
+}  // namespace mg
