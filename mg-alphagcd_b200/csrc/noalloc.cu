@@ -3,17 +3,25 @@
 // Some callers cannot call cudaMalloc: a serving process that has handed its
 // whole HBM budget to its own pool, or code that must not enter the CUDA
 // allocator at all.  mg_local_move_noalloc gives them one local-move sweep on
-// a graph they already hold in device memory.  The per-block hash tables,
-// which every other sweep path takes from engine-owned allocations, live
-// here in a fixed file-scope device array of kNoAllocScratchBytes.  Each
-// block processes vertices in turn with its own slice of that array (room for
-// pow2(2 * max degree + 2) slots); a vertex uses only the first
-// pow2(2 * its degree + 2) slots of it as an open-addressing table, so the
-// work per vertex follows its own degree, not the graph's maximum.  The arithmetic is the
-// engine's FP64 gain (same tie-break, same version 1 / 2 rules), so for
-// integral weights the result equals mg_local_move exactly.
+// a graph they already hold in device memory.  There is no room for lists of
+// vertices by degree, so every kernel walks all vertices and takes those of
+// its degrees:
+//   <= 32       8 lanes per vertex, <= 256 a warp: tables in shared memory
+//   <= 2,048    256 threads per vertex, <= 10,922 a 1,024-thread CTA: the same
+//   larger      a CTA per vertex, tables in a fixed file-scope device array of
+//               kNoAllocScratchBytes (room for pow2(2 * max degree + 2) slots
+//               per CTA)
+// The kernels of degrees that the graph does not have are not launched.  A
+// vertex uses only the first pow2 >= 2 * its degree slots of its table and
+// leaves them empty, so the work per vertex follows its own degree.  Threads
+// per vertex follow the degree because most vertices have few edges: 256
+// threads for each vertex took 29.8 ms on 500,009 vertices with 9.9 M entries
+// (integer weights, degrees up to 1.4e4).
+// The arithmetic is the engine's FP64 gain (same tie-break, same version 1 / 2
+// rules), so for integral weights the result equals mg_local_move exactly.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "handles.cuh"
 
@@ -62,99 +70,308 @@ __device__ __forceinline__ bool nb_better(double g2, uint32_t c2, double g1, uin
     return g2 > g1 || (g2 == g1 && (up ? c2 < c1 : c2 > c1));
 }
 
-__global__ void __launch_bounds__(kNoAllocThreads) noalloc_move_kernel(NoAllocArgs A, uint32_t *tkeys,
-                                                                       double *tvals, uint32_t tsize) {
-    __shared__ double red_e[kNoAllocThreads / 32];
-    __shared__ double red_g[kNoAllocThreads / 32];
-    __shared__ uint32_t red_c[kNoAllocThreads / 32];
-    uint32_t *keys = tkeys + (size_t)blockIdx.x * tsize;
-    double *vals = tvals + (size_t)blockIdx.x * tsize;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t v = blockIdx.x; v < A.n; v += gridDim.x) {
-        const uint32_t src = A.C[v];
-        const double ki = A.k[v];
-        const double a = A.sigma[src] - ki;
-        const uint32_t lo = A.off[v], hi = A.off[v + 1];
-        // this vertex's table: the first ts slots of the block's slice, a
-        // power of two >= 2 * degree + 2 (load <= 1/2); every slot it touches
-        // lies below ts and is cleaned by its evaluation loop
-        uint32_t ts = 32;
-        while (ts < 2 * (hi - lo) + 2 && ts < tsize) ts <<= 1;
-        double e_part = 0;
-        for (uint32_t e = lo + threadIdx.x; e < hi; e += kNoAllocThreads) {
-            const uint32_t j = A.col[e];
-            const uint32_t c = A.C[j];
-            const double w = A.w ? A.w[e] : 1.0;
-            if (c != src) {
-                const bool cand = A.version == 1 ? (A.up ? c < src : c > src) : true;
-                if (!cand) continue;
-                uint32_t s = hash_range(c, ts);
-                for (uint32_t p = 0; p < ts; p++) {
-                    uint32_t cur = ((volatile uint32_t *)keys)[s];
-                    if (cur == c) break;
-                    if (cur == kEmpty) {
-                        uint32_t prev = atomicCAS(keys + s, kEmpty, c);
-                        if (prev == kEmpty || prev == c) break;
-                    }
-                    s = s + 1 == ts ? 0 : s + 1;
-                }
-                atomicAdd(vals + s, w);
-            } else if (j != v) {
-                e_part += w;  // self-loops (j == v) stay out of e_src
+// table value: unit weights count in 32 bits, others add in double
+template <bool UNIT>
+using NbVal = typename std::conditional<UNIT, uint32_t, double>::type;
+template <bool UNIT>
+__device__ __forceinline__ NbVal<UNIT> nb_weight(const NoAllocArgs &A, uint32_t e) {
+    if constexpr (UNIT) return 1u;
+    else return A.w[e];
+}
+__device__ __forceinline__ double nb_double(uint32_t x) { return u2d(x); }
+__device__ __forceinline__ double nb_double(double x) { return x; }
+
+// log2 of the slots of a vertex of degree d: at least 2 * d and 16, at most 2^most
+__device__ __forceinline__ int nb_bits(uint32_t d, int most) {
+    const int want = d <= 8 ? 4 : 33 - __clz(2 * d - 1);
+    return want < most ? want : most;
+}
+
+__device__ __forceinline__ double nb_gain(const NoAllocArgs &A, double kic, double e_src, double ki, double a,
+                                          double sc) {
+    double t = __dmul_rn(ki, __dsub_rn(a, sc));
+    t = div_by(t, A.two_m, A.r_two_m);
+    t = __dsub_rn(e_src, t);
+    return div_by(__dsub_rn(kic, t), A.m, A.r_m);
+}
+
+__device__ __forceinline__ uint32_t nb_final(const NoAllocArgs &A, uint32_t dst, uint32_t src) {
+    if (A.version == 1) return dst;
+    return A.up ? (dst < src ? dst : src) : (dst > src ? dst : src);
+}
+
+// The edges t, t + GT, ... of vertex v into its table; returns the thread's
+// part of e.  Four edges in flight per thread.
+template <int GT, bool UNIT>
+__device__ __forceinline__ NbVal<UNIT> nb_insert(const NoAllocArgs &A, uint32_t v, uint32_t lo, uint32_t hi,
+                                                 uint32_t src, uint32_t t, uint32_t *keys, NbVal<UNIT> *vals,
+                                                 int bits) {
+    using V = NbVal<UNIT>;
+    const uint32_t mask = (1u << bits) - 1u;
+    V e_part = V(0);
+    for (uint32_t base = lo + t; base < hi; base += 4 * GT) {
+        uint32_t j[4], c[4];
+        V w[4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const uint32_t e = base + b * GT;
+            j[b] = e < hi ? A.col[e] : kEmpty;
+            w[b] = e < hi ? nb_weight<UNIT>(A, e) : V(0);
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++) c[b] = j[b] != kEmpty ? A.C[j[b]] : kEmpty;
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            if (j[b] == kEmpty) continue;
+            if (c[b] == src) {
+                if (j[b] != v) e_part += w[b];  // self-loops (j == v) stay out of e_src
+                continue;
+            }
+            if (A.version == 1 && !(A.up ? c[b] < src : c[b] > src)) continue;
+            uint32_t s = hash_slot(c[b], bits);
+            for (uint32_t p = 0; p <= mask; p++) {
+                const uint32_t prev = atomicCAS(keys + s, kEmpty, c[b]);
+                if (prev == kEmpty || prev == c[b]) break;
+                s = (s + 1) & mask;
+            }
+            atomicAdd(vals + s, w[b]);
+        }
+    }
+    return e_part;
+}
+
+// The thread's best of the table's slots t, t + GT, ..., which it empties.
+template <int GT, bool UNIT>
+__device__ __forceinline__ void nb_evaluate(const NoAllocArgs &A, double e_src, double ki, double a, uint32_t t,
+                                            uint32_t *keys, NbVal<UNIT> *vals, int bits, double &best, uint32_t &dst) {
+    const uint32_t ts = 1u << bits;
+    for (uint32_t s0 = t; s0 < ts; s0 += 4 * GT) {
+        uint32_t c[4];
+        double kic[4], sc[4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const uint32_t s = s0 + b * GT;
+            c[b] = s < ts ? keys[s] : kEmpty;
+            if (c[b] != kEmpty) {
+                kic[b] = nb_double(vals[s]);
+                keys[s] = kEmpty;
+                vals[s] = 0;
             }
         }
-        e_part = warp_sum(e_part);
-        if (lane == 0) red_e[warp] = e_part;
-        __syncthreads();
-        double e_src = 0;
-        for (int i = 0; i < kNoAllocThreads / 32; i++) e_src += red_e[i];
-        double best = 0.0;
-        uint32_t dst = src;
-        for (uint32_t s = threadIdx.x; s < ts; s += kNoAllocThreads) {
-            const uint32_t c = keys[s];
-            if (c == kEmpty) continue;
-            const double kic = vals[s];
-            keys[s] = kEmpty;
-            vals[s] = 0.0;
-            double t = __dmul_rn(ki, __dsub_rn(a, A.sigma[c]));
-            t = div_by(t, A.two_m, A.r_two_m);
-            t = __dsub_rn(e_src, t);
-            const double g = div_by(__dsub_rn(kic, t), A.m, A.r_m);
-            if (nb_better(g, c, best, dst, A.up)) {
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+            if (c[b] != kEmpty) sc[b] = A.sigma[c[b]];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            if (c[b] == kEmpty) continue;
+            const double g = nb_gain(A, kic[b], e_src, ki, a, sc[b]);
+            if (nb_better(g, c[b], best, dst, A.up)) {
                 best = g;
-                dst = c;
+                dst = c[b];
             }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            double g2 = __shfl_xor_sync(0xffffffffu, best, o);
-            uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-            if (nb_better(g2, c2, best, dst, A.up)) {
-                best = g2;
-                dst = c2;
-            }
+    }
+}
+
+// One vertex by GT <= 32 lanes of a warp (mask: those lanes).
+template <int GT, bool UNIT>
+__device__ __forceinline__ void nb_vertex(const NoAllocArgs &A, uint32_t v, uint32_t lo, uint32_t hi, uint32_t lanes,
+                                          uint32_t *keys, NbVal<UNIT> *vals, int most) {
+    const uint32_t t = threadIdx.x & (GT - 1);
+    const uint32_t src = A.C[v];
+    const double ki = A.k[v];
+    const int bits = nb_bits(hi - lo, most);
+    NbVal<UNIT> e = nb_insert<GT, UNIT>(A, v, lo, hi, src, t, keys, vals, bits);
+    __syncwarp(lanes);
+#pragma unroll
+    for (int o = GT / 2; o > 0; o >>= 1) e += __shfl_xor_sync(lanes, e, o);
+    const double a = A.sigma[src] - ki;
+    double best = 0.0;
+    uint32_t dst = src;
+    nb_evaluate<GT, UNIT>(A, nb_double(e), ki, a, t, keys, vals, bits, best, dst);
+#pragma unroll
+    for (int o = GT / 2; o > 0; o >>= 1) {
+        const double g2 = __shfl_xor_sync(lanes, best, o);
+        const uint32_t c2 = __shfl_xor_sync(lanes, dst, o);
+        if (nb_better(g2, c2, best, dst, A.up)) {
+            best = g2;
+            dst = c2;
         }
-        __syncthreads();  // everyone has read red_e before it is reused
-        if (lane == 0) {
-            red_g[warp] = best;
-            red_c[warp] = dst;
+    }
+    if (t == 0) A.C_new[v] = nb_final(A, dst, src);
+    __syncwarp(lanes);  // the table is empty before the next vertex
+}
+
+// Degrees up to kWarpDeg: a warp takes 32 consecutive vertices, first those of
+// at most kLaneDeg edges, four at a time by 8 lanes, then the others.
+// 4 blocks of 256 threads per SM (48 KB of tables each).
+constexpr uint32_t kLaneDeg = 32, kWarpDeg = 256, kGroupDeg = 2048, kCtaDeg = 10922;
+constexpr int kWarpBits = 9, kGroupBits = 12, kCtaBits = 14;
+constexpr int kCtaThreads = 1024;
+
+template <bool UNIT>
+__global__ void __launch_bounds__(kNoAllocThreads, 4) noalloc_warp_kernel(NoAllocArgs A) {
+    using V = NbVal<UNIT>;
+    constexpr uint32_t S = 1u << kWarpBits;
+    extern __shared__ __align__(16) unsigned char nb_smem[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    V *vals = (V *)nb_smem + warp * S;
+    uint32_t *keys = (uint32_t *)(nb_smem + sizeof(V) * S * (kNoAllocThreads / 32)) + warp * S;
+    for (uint32_t s = lane; s < S; s += 32) {
+        keys[s] = kEmpty;
+        vals[s] = V(0);
+    }
+    __syncwarp();
+    const uint32_t tile = lane / 8, lanes = 0xffu << (8 * tile);
+    const uint64_t step = (uint64_t)gridDim.x * kNoAllocThreads;
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kNoAllocThreads + 32 * warp; v0 < A.n; v0 += step) {
+        const uint64_t v = v0 + lane;
+        const uint32_t lo = v < A.n ? A.off[v] : 0u, hi = v < A.n ? A.off[v + 1] : 0u;
+        const uint32_t d = hi - lo;
+        // one tile's slice: a quarter of the warp's
+        for (uint32_t r = 0; r < 32; r += 4) {
+            const uint32_t q = r + tile;
+            const uint32_t vd = __shfl_sync(0xffffffffu, d, q), vlo = __shfl_sync(0xffffffffu, lo, q);
+            if (v0 + q < A.n && vd <= kLaneDeg)
+                nb_vertex<8, UNIT>(A, (uint32_t)v0 + q, vlo, vlo + vd, lanes, keys + tile * (S / 4),
+                                   vals + tile * (S / 4), kWarpBits - 2);
+            __syncwarp();
+        }
+        uint32_t rest = __ballot_sync(0xffffffffu, v < A.n && d > kLaneDeg && d <= kWarpDeg);
+        for (; rest; rest &= rest - 1) {
+            const uint32_t q = __ffs(rest) - 1;
+            const uint32_t vd = __shfl_sync(0xffffffffu, d, q), vlo = __shfl_sync(0xffffffffu, lo, q);
+            nb_vertex<32, UNIT>(A, (uint32_t)v0 + q, vlo, vlo + vd, 0xffffffffu, keys, vals, kWarpBits);
+        }
+    }
+}
+
+// One vertex by a CTA of NT threads.
+template <int NT, bool UNIT>
+__device__ __forceinline__ void nb_cta_vertex(const NoAllocArgs &A, uint32_t v, uint32_t *keys, NbVal<UNIT> *vals,
+                                              int most, double *red_g, uint32_t *red_c) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lo = A.off[v], hi = A.off[v + 1], src = A.C[v];
+    const double ki = A.k[v];
+    const int bits = nb_bits(hi - lo, most);
+    const double ep = warp_sum(
+        nb_double(nb_insert<NT, UNIT>(A, v, lo, hi, src, threadIdx.x, keys, vals, bits)));
+    if (lane == 0) red_g[warp] = ep;
+    __syncthreads();
+    double e_src = 0;
+    for (int i = 0; i < NT / 32; i++) e_src += red_g[i];
+    const double a = A.sigma[src] - ki;
+    double best = 0.0;
+    uint32_t dst = src;
+    nb_evaluate<NT, UNIT>(A, e_src, ki, a, threadIdx.x, keys, vals, bits, best, dst);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double g2 = __shfl_xor_sync(0xffffffffu, best, o);
+        const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
+        if (nb_better(g2, c2, best, dst, A.up)) {
+            best = g2;
+            dst = c2;
+        }
+    }
+    __syncthreads();  // everyone has read red_g
+    if (lane == 0) {
+        red_g[warp] = best;
+        red_c[warp] = dst;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < NT / 32; i++)
+            if (nb_better(red_g[i], red_c[i], best, dst, A.up)) {
+                best = red_g[i];
+                dst = red_c[i];
+            }
+        A.C_new[v] = nb_final(A, dst, src);
+    }
+    __syncthreads();  // the table is empty, red_* are read
+}
+
+// The vertices of degrees in (dmin, dmax], a CTA each.  A CTA looks at NT
+// vertices at a time, eight consecutive ones (a sector of offsets) from each
+// of NT / 8 places spread over the ids, so that hubs with neighbouring ids
+// fall to different CTAs.  GLOBAL: the tables are the CTA's part of the scratch
+// array (cleared by the host), else shared memory.
+template <int NT, bool UNIT, bool GLOBAL>
+__global__ void __launch_bounds__(NT) noalloc_cta_kernel(NoAllocArgs A, uint32_t dmin, uint32_t dmax, int most,
+                                                         uint32_t *tkeys, double *tvals) {
+    using V = NbVal<UNIT>;
+    extern __shared__ __align__(16) unsigned char nb_smem[];
+    __shared__ double red_g[NT / 32];
+    __shared__ uint32_t red_c[NT / 32];
+    __shared__ uint32_t list[NT], count;
+    const uint32_t S = 1u << most;
+    V *vals = GLOBAL ? (V *)(tvals + (size_t)blockIdx.x * S) : (V *)nb_smem;
+    uint32_t *keys = GLOBAL ? tkeys + (size_t)blockIdx.x * S : (uint32_t *)(nb_smem + sizeof(V) * S);
+    if constexpr (!GLOBAL) {
+        for (uint32_t s = threadIdx.x; s < S; s += NT) {
+            keys[s] = kEmpty;
+            vals[s] = V(0);
+        }
+    }
+    const uint32_t eights = (uint32_t)(((uint64_t)A.n + 7) / 8), rounds = (eights + NT / 8 - 1) / (NT / 8);
+    for (uint32_t r = blockIdx.x; r < rounds; r += gridDim.x) {
+        if (threadIdx.x == 0) count = 0;
+        __syncthreads();
+        const uint64_t v = ((uint64_t)r + (uint64_t)(threadIdx.x / 8) * rounds) * 8 + threadIdx.x % 8;
+        if (v < A.n) {
+            const uint32_t d = A.off[v + 1] - A.off[v];
+            if (d > dmin && d <= dmax) list[atomicAdd(&count, 1u)] = (uint32_t)v;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int i = 0; i < kNoAllocThreads / 32; i++)
-                if (nb_better(red_g[i], red_c[i], best, dst, A.up)) {
-                    best = red_g[i];
-                    dst = red_c[i];
-                }
-            uint32_t out = dst;
-            if (A.version != 1) out = A.up ? (dst < src ? dst : src) : (dst > src ? dst : src);
-            A.C_new[v] = out;
-        }
-        __syncthreads();  // table reset and red_* reads complete before the next vertex
+        const uint32_t cnt = count;
+        for (uint32_t i = 0; i < cnt; i++) nb_cta_vertex<NT, UNIT>(A, list[i], keys, vals, most, red_g, red_c);
+        __syncthreads();
     }
 }
 
 std::mutex g_noalloc_mu;
 void *g_noalloc_addr[kMaxDevices] = {nullptr};
+
+template <bool UNIT>
+constexpr size_t nb_smem_bytes(int bits, int tables) {
+    return ((sizeof(NbVal<UNIT>) + sizeof(uint32_t)) * (size_t)tables) << bits;
+}
+
+// shared-memory limits of the kernels, per device
+template <bool UNIT>
+cudaError_t nb_set_limits() {
+    cudaError_t e = cudaFuncSetAttribute(noalloc_warp_kernel<UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)nb_smem_bytes<UNIT>(kWarpBits, kNoAllocThreads / 32));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(noalloc_cta_kernel<kNoAllocThreads, UNIT, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nb_smem_bytes<UNIT>(kGroupBits, 1));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(noalloc_cta_kernel<kCtaThreads, UNIT, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nb_smem_bytes<UNIT>(kCtaBits, 1));
+    return e;
+}
+
+template <bool UNIT>
+void nb_launch(const NoAllocArgs &A, uint32_t maxdeg, uint32_t blocks, uint32_t tsize, uint32_t *tkeys, double *tvals,
+               cudaStream_t s) {
+    if (maxdeg > kCtaDeg) {
+        // the scratch keeps the previous call's contents: clear the tables
+        noalloc_clear_kernel<<<148 * 4, 256, 0, s>>>(tkeys, tvals, (size_t)blocks * tsize);
+        noalloc_cta_kernel<kCtaThreads, UNIT, true>
+            <<<blocks, kCtaThreads, 0, s>>>(A, kCtaDeg, 0xFFFFFFFFu, 31 - __builtin_clz(tsize), tkeys, tvals);
+    }
+    const uint32_t eights = (uint32_t)ceil_div(A.n, 8);
+    if (maxdeg > kGroupDeg)
+        noalloc_cta_kernel<kCtaThreads, UNIT, false>
+            <<<std::min<uint32_t>(148, (eights + kCtaThreads / 8 - 1) / (kCtaThreads / 8)), kCtaThreads,
+               nb_smem_bytes<UNIT>(kCtaBits, 1), s>>>(A, kGroupDeg, kCtaDeg, kCtaBits, nullptr, nullptr);
+    if (maxdeg > kWarpDeg)
+        noalloc_cta_kernel<kNoAllocThreads, UNIT, false>
+            <<<std::min<uint32_t>(148 * 4, (eights + kNoAllocThreads / 8 - 1) / (kNoAllocThreads / 8)), kNoAllocThreads,
+               nb_smem_bytes<UNIT>(kGroupBits, 1), s>>>(A, kWarpDeg, kGroupDeg, kGroupBits, nullptr, nullptr);
+    noalloc_warp_kernel<UNIT>
+        <<<(unsigned)std::min<uint64_t>(148 * 4, ceil_div(A.n, kNoAllocThreads)), kNoAllocThreads,
+           nb_smem_bytes<UNIT>(kWarpBits, kNoAllocThreads / 32), s>>>(A);
+}
 
 mg_status noalloc_fail(mg_status st, const std::string &msg) {
     set_orphan_error("mg_local_move_noalloc: " + msg);
@@ -182,10 +399,12 @@ extern "C" mg_status mg_local_move_noalloc(uint32_t n, const uint32_t *d_offsets
         // static array (its host-side name is only a stand-in)
         std::lock_guard<std::mutex> lock(g_noalloc_mu);
         if (!g_noalloc_addr[dev]) {
-            cudaError_t e = cudaGetSymbolAddress(&g_noalloc_addr[dev], g_noalloc_scratch);
+            cudaError_t e = nb_set_limits<true>();
+            if (e == cudaSuccess) e = nb_set_limits<false>();
+            if (e == cudaSuccess) e = cudaGetSymbolAddress(&g_noalloc_addr[dev], g_noalloc_scratch);
             if (e != cudaSuccess) {
                 g_noalloc_addr[dev] = nullptr;
-                return noalloc_fail(MG_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
+                return noalloc_fail(MG_ERR_CUDA, std::string("device set-up: ") + cudaGetErrorString(e));
             }
         }
         base = g_noalloc_addr[dev];
@@ -205,12 +424,10 @@ extern "C" mg_status mg_local_move_noalloc(uint32_t n, const uint32_t *d_offsets
     if (table_bytes > room)
         return noalloc_fail(MG_ERR_UNSUPPORTED, "max degree " + std::to_string(maxdeg) +
                                                     " needs a table larger than the static scratch (16 MiB)");
-    uint32_t blocks = (uint32_t)std::min<size_t>({room / table_bytes, (size_t)148 * 4, (size_t)n});
+    // CTAs of the degrees above kCtaDeg
+    const uint32_t blocks = (uint32_t)std::min<size_t>({room / table_bytes, (size_t)148, (size_t)n});
     uint32_t *tkeys = (uint32_t *)((unsigned char *)base + 256);
     double *tvals = (double *)((unsigned char *)base + 256 + (((size_t)blocks * tsize * sizeof(uint32_t) + 255) & ~(size_t)255));
-    const size_t slots = (size_t)blocks * tsize;
-    // the array keeps the previous call's contents: clear the tables
-    noalloc_clear_kernel<<<148 * 4, 256, 0, s>>>(tkeys, tvals, slots);
     NoAllocArgs A;
     A.off = d_offsets;
     A.col = d_cols;
@@ -226,7 +443,8 @@ extern "C" mg_status mg_local_move_noalloc(uint32_t n, const uint32_t *d_offsets
     A.r_two_m = 1.0 / A.two_m;
     A.version = version;
     A.up = up ? 1 : 0;
-    noalloc_move_kernel<<<blocks, kNoAllocThreads, 0, s>>>(A, tkeys, tvals, tsize);
+    if (d_weights) nb_launch<false>(A, maxdeg, blocks, tsize, tkeys, tvals, s);
+    else nb_launch<true>(A, maxdeg, blocks, tsize, tkeys, tvals, s);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(MG_ERR_CUDA, cudaGetErrorString(e));
     return MG_OK;
