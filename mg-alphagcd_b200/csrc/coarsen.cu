@@ -391,6 +391,14 @@ inline unsigned grid_for(uint64_t n, int threads = 256, uint64_t cap = 148ull * 
     return (unsigned)(g ? g : 1);
 }
 
+// A count from the device, through pinned memory; waits for the stream.
+uint32_t read_count(const uint32_t *d, CoarsenWorkspace &ws, cudaStream_t s) {
+    uint32_t *h = ws.prim.pinned();
+    MG_CUDA(cudaMemcpyAsync(h, d, sizeof *h, cudaMemcpyDeviceToHost, s));
+    MG_CUDA(cudaStreamSynchronize(s));
+    return *h;
+}
+
 void emit_rows(const uint64_t *ukey, uint32_t u, int bc, uint32_t n_rows, uint32_t *off, uint32_t *col,
                cudaStream_t s) {
     emit_cols_kernel<<<grid_for(u), 256, 0, s>>>(ukey, u, bc, col);
@@ -407,9 +415,7 @@ uint32_t unique_runs(const uint64_t *keys, size_t m, int bc, uint32_t n_rows, Le
     run_heads_kernel<<<grid_for(m), 256, 0, s>>>(keys, m, head);
     MG_LAUNCH_CHECK();
     exclusive_scan<uint32_t>(head, seg, m, seg + m, s, ws.prim);
-    uint32_t u = 0;
-    MG_CUDA(cudaMemcpyAsync(&u, seg + m, sizeof u, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
+    const uint32_t u = read_count(seg + m, ws, s);
     uint64_t *ukey = ws.u64tmp.ensure(u + 1);
     uint32_t *ustart = ws.u32tmp.ensure(u + 1);
     compact_runs_kernel<<<grid_for(m), 256, 0, s>>>(keys, m, head, seg, ukey, ustart);
@@ -599,9 +605,7 @@ uint32_t unique_runs_tiled(const uint64_t *keys, size_t m, int bc, uint32_t n_ro
     run_count_kernel<<<grid, kRunThreads, 0, s>>>(keys, m, tcount);
     MG_LAUNCH_CHECK();
     exclusive_scan<uint32_t>(tcount, tcount, tiles, tcount + tiles, s, ws.prim);
-    uint32_t u = 0;
-    MG_CUDA(cudaMemcpyAsync(&u, tcount + tiles, sizeof u, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
+    const uint32_t u = read_count(tcount + tiles, ws, s);
     uint32_t *ustart = ws.u32tmp.ensure((size_t)u + 1);
     out.n = n_rows;
     out.nnz = u;
@@ -650,10 +654,7 @@ uint32_t relabel_dense(const uint32_t *C, uint32_t n, uint32_t *C_dense, Coarsen
     exclusive_scan<uint32_t>(flags, newid, n, newid + n, s, ws.prim);
     apply_relabel_kernel<<<grid_for(n), 256, 0, s>>>(C, n, newid, C_dense);
     MG_LAUNCH_CHECK();
-    uint32_t nn = 0;
-    MG_CUDA(cudaMemcpyAsync(&nn, newid + n, sizeof nn, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
-    return nn;
+    return read_count(newid + n, ws, s);
 }
 
 void coarsen_level(const GraphView &g, const uint32_t *Cd, uint32_t n_new, int integral, LevelGraph &out,
@@ -743,9 +744,7 @@ void coarsen_level(const GraphView &g, const uint32_t *Cd, uint32_t n_new, int i
         if (ipay) expand(ivals, std::true_type(), std::false_type());
         else expand(vals, std::true_type(), std::false_type());
         exclusive_scan<uint32_t>(tcount, tcount, tiles, tcount + tiles, s, ws.prim);
-        uint32_t d = 0;
-        MG_CUDA(cudaMemcpyAsync(&d, tcount + tiles, sizeof d, cudaMemcpyDeviceToHost, s));
-        MG_CUDA(cudaStreamSynchronize(s));
+        const uint32_t d = read_count(tcount + tiles, ws, s);
         const unsigned gc = grid_for(tiles, 1, 148ull * 16);
         if (ipay) compact_tiles_kernel<uint32_t><<<gc, 256, 0, s>>>(keys, ivals, tcount, tiles, keys2, ivals2);
         else compact_tiles_kernel<double><<<gc, 256, 0, s>>>(keys, vals, tcount, tiles, keys2, vals2);

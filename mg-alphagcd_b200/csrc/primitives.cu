@@ -54,11 +54,21 @@ __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const T *in, 
     if (threadIdx.x == 0) sums[blockIdx.x] = (uint64_t)tot;
 }
 
-template <class T>
+// SUMS: offs holds the tiles' sums and the block adds up those before its own
+// (which saves the launches that scan them; few tiles only).  Else offs holds
+// the tiles' offsets.
+template <class T, bool SUMS>
 __global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const T *in, T *out, size_t n,
                                                                    const uint64_t *offs, T *d_total) {
     __shared__ T sw[8];
     __shared__ T tot;
+    __shared__ uint64_t before;
+    if constexpr (SUMS) {
+        __shared__ uint64_t sw64[8];
+        uint64_t sum = 0;
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) sum += offs[b];
+        block_exclusive_sum<uint64_t>(sum, sw64, &before);
+    }
     size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
     T v[kScanItems];
     T acc = 0;
@@ -69,7 +79,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const T *in, T 
         acc += v[k];
     }
     T ex = block_exclusive_sum<T>(acc, sw, &tot);
-    T run = (T)offs[blockIdx.x] + ex;
+    T run = (T)(SUMS ? before : offs[blockIdx.x]) + ex;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
         size_t i = base + k;
@@ -79,12 +89,64 @@ __global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const T *in, T 
     if (d_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) *d_total = run;
 }
 
+// One block, n <= kScanOne: the whole scan in one launch.
+constexpr int kScanOneThreads = 1024;
+constexpr int kScanOne = kScanOneThreads * 8;
+template <class T>
+__global__ void __launch_bounds__(kScanOneThreads) scan_one_kernel(const T *in, T *out, uint32_t n, T *d_total) {
+    __shared__ T wsum[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t base = threadIdx.x * 8;
+    T v[8], acc = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        v[k] = base + k < n ? in[base + k] : T(0);
+        acc += v[k];
+    }
+    T incl = acc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    T run = incl - acc;
+    for (uint32_t w = 0; w < warp; w++) run += wsum[w];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        if (base + k < n) out[base + k] = run;
+        run += v[k];
+    }
+    if (d_total && threadIdx.x == kScanOneThreads - 1) *d_total = run;
+}
+
+// Tiles whose sums each block adds up itself (2 MB of reads over all blocks).
+constexpr size_t kScanSumTiles = 512;
+
 }  // namespace
 
+uint32_t *PrimWorkspace::pinned() {
+    if (!h_small) MG_CUDA(cudaMallocHost(&h_small, kPinnedWords * sizeof(uint32_t)));
+    return h_small;
+}
+PrimWorkspace::~PrimWorkspace() {
+    if (h_small) cudaFreeHost(h_small);
+}
+
+// Launches by size: one block up to 8,192 items, a sum and a scan per tile up
+// to 512 tiles (1 M items), else the tiles' sums are scanned between the two.
+// Scans of a level's counts, offsets and histograms are mostly of the first
+// two kinds, and a launch costs as much as such a scan (3 us).
 template <class T>
 static void scan_level(const T *in, T *out, size_t n, T *d_total, cudaStream_t s, PrimWorkspace &ws, int depth) {
     if (n == 0) {
         if (d_total) MG_CUDA(cudaMemsetAsync(d_total, 0, sizeof(T), s));
+        return;
+    }
+    if (n <= kScanOne) {
+        scan_one_kernel<T><<<1, kScanOneThreads, 0, s>>>(in, out, (uint32_t)n, d_total);
+        MG_LAUNCH_CHECK();
         return;
     }
     size_t tiles = ceil_div(n, kScanTile);
@@ -93,9 +155,12 @@ static void scan_level(const T *in, T *out, size_t n, T *d_total, cudaStream_t s
     uint64_t *bs = sums.ensure(tiles + 1);
     scan_reduce_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, bs);
     MG_LAUNCH_CHECK();
-    if (tiles > 1) scan_level<uint64_t>(bs, bs, tiles, nullptr, s, ws, depth + 1);
-    else MG_CUDA(cudaMemsetAsync(bs, 0, sizeof(uint64_t), s));
-    scan_down_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, bs, d_total);
+    if (tiles <= kScanSumTiles) {
+        scan_down_kernel<T, true><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, bs, d_total);
+    } else {
+        scan_level<uint64_t>(bs, bs, tiles, nullptr, s, ws, depth + 1);
+        scan_down_kernel<T, false><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, bs, d_total);
+    }
     MG_LAUNCH_CHECK();
 }
 
@@ -221,6 +286,112 @@ __global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(const uint64_t *
     }
 }
 
+// All passes of a sort of at most kRsOne keys in one block: the keys stay in
+// registers and shared memory between passes.  Ranks as in the scatter kernel
+// (a warp owns 256 consecutive positions, visited in lane order), so stable.
+// A level of a few thousand entries is sorted in one launch of about 8 us a
+// pass instead of three or four launches a pass.
+constexpr int kRsOneThreads = 1024, kRsOneWarps = kRsOneThreads / 32, kRsOneRounds = 8;
+constexpr int kRsOne = kRsOneThreads * kRsOneRounds;
+// counters by digit and warp, a row of 33 per digit (a warp's lanes, which hold
+// different digits, then fall on different banks)
+constexpr int kRsOneRow = kRsOneWarps + 1, kRsOneCnt = 256 * kRsOneRow;
+
+template <class V>
+constexpr size_t rs_one_smem() {
+    return (size_t)kRsOne * (sizeof(uint64_t) + (std::is_same<V, NoVal>::value ? 0 : sizeof(V))) +
+           (size_t)kRsOneCnt * sizeof(uint32_t);
+}
+
+template <class V>
+__global__ void __launch_bounds__(kRsOneThreads) rs_one_kernel(const uint64_t *keys, const V *vals, uint64_t *okeys,
+                                                               V *ovals, uint32_t n, int lo_bit, int bits) {
+    constexpr bool HasV = !std::is_same<V, NoVal>::value;
+    extern __shared__ __align__(16) unsigned char rs_smem[];
+    uint64_t *sk = (uint64_t *)rs_smem;
+    uint32_t *cnt = (uint32_t *)(rs_smem + sizeof(uint64_t) * kRsOne);  // [digit][warp], padded
+    V *sv = (V *)(rs_smem + sizeof(uint64_t) * kRsOne + sizeof(uint32_t) * kRsOneCnt);
+    __shared__ uint32_t wsum[kRsOneWarps];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    const uint32_t wbase = warp * (kRsOneRounds * 32), lt = (1u << lane) - 1u;
+    uint64_t k[kRsOneRounds];
+    V v[HasV ? kRsOneRounds : 1];
+#pragma unroll
+    for (int r = 0; r < kRsOneRounds; r++) {
+        const uint32_t i = wbase + r * 32 + lane;
+        k[r] = i < n ? keys[i] : ~0ull;
+        if constexpr (HasV) v[r] = i < n ? vals[i] : V();
+    }
+    for (int shift = lo_bit; shift < bits; shift += 8) {
+        for (uint32_t d = t; d < kRsOneCnt; d += kRsOneThreads) cnt[d] = 0;
+        __syncthreads();
+        uint32_t rank[kRsOneRounds];
+#pragma unroll
+        for (int r = 0; r < kRsOneRounds; r++) {
+            const uint32_t i = wbase + r * 32 + lane;
+            const uint32_t d = i < n ? (uint32_t)((k[r] >> shift) & 0xFF) : 0x100u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t before = __popc(peers & lt);
+            const uint32_t run = d < 256 ? cnt[d * kRsOneRow + warp] : 0u;
+            rank[r] = run + before;
+            __syncwarp();
+            if (d < 256 && before == 0) cnt[d * kRsOneRow + warp] = run + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        // exclusive prefix over (digit, warp): 8 counters per thread
+        uint32_t *mine = cnt + (t >> 2) * kRsOneRow + (t & 3u) * 8;
+        uint32_t c[8], acc = 0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            c[q] = acc;
+            acc += mine[q];
+        }
+        uint32_t incl = acc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        uint32_t before = incl - acc;
+        for (uint32_t w = 0; w < warp; w++) before += wsum[w];
+#pragma unroll
+        for (int q = 0; q < 8; q++) mine[q] = before + c[q];
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRsOneRounds; r++) {
+            const uint32_t i = wbase + r * 32 + lane;
+            if (i < n) {
+                const uint32_t pos = cnt[(uint32_t)((k[r] >> shift) & 0xFF) * kRsOneRow + warp] + rank[r];
+                sk[pos] = k[r];
+                if constexpr (HasV) sv[pos] = v[r];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRsOneRounds; r++) {
+            const uint32_t i = wbase + r * 32 + lane;
+            if (i < n) {
+                k[r] = sk[i];
+                if constexpr (HasV) v[r] = sv[i];
+            }
+        }
+        // (the counters are cleared behind the next pass's barrier; the keys'
+        // slots are written again only after it)
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < kRsOneRounds; r++) {
+        const uint32_t i = wbase + r * 32 + lane;
+        if (i < n) {
+            okeys[i] = k[r];
+            if constexpr (HasV) ovals[i] = v[r];
+        }
+    }
+}
+
 }  // namespace
 
 template <class V>
@@ -228,6 +399,14 @@ bool radix_sort(uint64_t *keys, V *vals, uint64_t *keys_alt, V *vals_alt, size_t
                 cudaStream_t s, PrimWorkspace &ws, int lo_bit) {
     if (n <= 1 || bits <= lo_bit) return false;
     MG_CHECK(n < 0xFFFFFFFFull, MG_ERR_UNSUPPORTED, "radix_sort: more than 2^32-1 keys");
+    if (n <= kRsOne) {
+        MG_CUDA(cudaFuncSetAttribute(rs_one_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)rs_one_smem<V>()));
+        rs_one_kernel<V><<<1, kRsOneThreads, rs_one_smem<V>(), s>>>(keys, vals, keys_alt, vals_alt, (uint32_t)n,
+                                                                     lo_bit, bits);
+        MG_LAUNCH_CHECK();
+        return true;
+    }
     uint32_t tiles = (uint32_t)ceil_div(n, kRsTile);
     uint32_t *hist = ws.hist.ensure((size_t)tiles * 256 + 1);
     uint64_t *ka = keys, *kb = keys_alt;

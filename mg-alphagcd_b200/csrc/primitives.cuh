@@ -17,7 +17,11 @@ struct PrimWorkspace {
     DBuf<uint64_t> scan_a, scan_b, scan_c;  // block sums of the scan levels
     DBuf<uint32_t> hist;                    // radix tile histograms
     DBuf<uint32_t> bins;                    // degree-bin block counts
+    uint32_t *h_small = nullptr;            // pinned words for counts read back
+    uint32_t *pinned();                     // kPinnedWords of them
+    ~PrimWorkspace();
 };
+constexpr int kPinnedWords = 64;
 
 // out[i] = sum_{j<i} in[i]; returns nothing (the total, when asked for, is
 // written to *d_total on the device).  in and out may alias.  T: uint32_t or
