@@ -179,6 +179,63 @@ __device__ __forceinline__ G shfl_xor_g(G v, int o) {
     return __shfl_xor_sync(0xffffffffu, v, o);
 }
 
+// Warp sums of table values: 32-bit integers in one warp-reduce instruction
+// (a shuffle tree takes five shuffles and five adds), doubles by shuffles.
+__device__ __forceinline__ uint32_t value_sum(uint32_t v) { return __reduce_add_sync(0xffffffffu, v); }
+__device__ __forceinline__ double value_sum(double v) { return warp_sum(v); }
+
+// The better candidate of a warp in the order of better(), in every lane.  A
+// running best starts at gain 0 and only grows, so it is never negative or NaN
+// and its bits, sign dropped (-0.0 counts as 0), order like unsigned integers:
+// the largest high word, the largest low word among its lanes, then the
+// smallest (up) or largest id among the lanes with both -- three warp-reduce
+// instructions where a shuffle tree takes fifteen shuffles and ten 64-bit
+// compares.
+__device__ __forceinline__ void warp_argmax_bits(uint32_t &hi, uint32_t &lo, uint32_t &dst, int up) {
+    const uint32_t mh = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t l = hi == mh ? lo : 0u;
+    const uint32_t ml = __reduce_max_sync(0xffffffffu, l);
+    const bool in = hi == mh && lo == ml;
+    dst = up ? __reduce_min_sync(0xffffffffu, in ? dst : 0xffffffffu) : __reduce_max_sync(0xffffffffu, in ? dst : 0u);
+    hi = mh;
+    lo = ml;
+}
+__device__ __forceinline__ void warp_argmax(double &best, uint32_t &dst, int up) {
+    uint32_t hi = (uint32_t)__double2hiint(best) & 0x7fffffffu, lo = (uint32_t)__double2loint(best);
+    warp_argmax_bits(hi, lo, dst, up);
+    best = __hiloint2double((int)hi, (int)lo);
+}
+__device__ __forceinline__ void warp_argmax(long long &best, uint32_t &dst, int up) {
+    uint32_t hi = (uint32_t)((unsigned long long)best >> 32), lo = (uint32_t)best;
+    warp_argmax_bits(hi, lo, dst, up);
+    best = (long long)(((unsigned long long)hi << 32) | lo);
+}
+__device__ __forceinline__ void warp_argmax(float &best, uint32_t &dst, int up) {
+    const uint32_t b = (uint32_t)__float_as_int(best) & 0x7fffffffu;
+    const uint32_t mb = __reduce_max_sync(0xffffffffu, b);
+    dst = up ? __reduce_min_sync(0xffffffffu, b == mb ? dst : 0xffffffffu)
+             : __reduce_max_sync(0xffffffffu, b == mb ? dst : 0u);
+    best = __int_as_float((int)mb);
+}
+
+// The same among the T lanes of a tile (a whole warp: the instructions above).
+template <int T, class G>
+__device__ __forceinline__ void tile_argmax(G &best, uint32_t &dst, int up) {
+    if constexpr (T == 32) {
+        warp_argmax(best, dst, up);
+    } else {
+#pragma unroll
+        for (int o = T / 2; o > 0; o >>= 1) {
+            const G g2 = shfl_xor_g(best, o);
+            const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
+            if (better(g2, c2, best, dst, up)) {
+                best = g2;
+                dst = c2;
+            }
+        }
+    }
+}
+
 // Block-level accumulation of sum_in / distinct into the sweep accumulators.
 __device__ __forceinline__ void flush_acc(SweepAcc *acc, int integral, double sin, unsigned dcnt) {
     __shared__ double s_f;
@@ -298,15 +355,7 @@ __global__ void __launch_bounds__(256) lm_tile_kernel(LMArgs A, uint32_t bin_off
             }
             dcnt++;
         }
-#pragma unroll
-        for (int o = T / 2; o > 0; o >>= 1) {
-            G g2 = shfl_xor_g(best, o);
-            uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-            if (better(g2, c2, best, dst, up)) {
-                best = g2;
-                dst = c2;
-            }
-        }
+        tile_argmax<T>(best, dst, up);
         if (active && gl == 0) {
             vv.N[i] = final_choice<VER>(dst, src, up);
             put_sin<BT>(A, i, sin, e_src + selfw);
@@ -334,15 +383,7 @@ __device__ __forceinline__ void group_sync() {
 // thread (the only one its callers read it from)
 template <int GT, class G>
 __device__ __forceinline__ void group_argmax(G &best, uint32_t &dst, int up, G *rg, uint32_t *rc) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        G g2 = shfl_xor_g(best, o);
-        uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-        if (better(g2, c2, best, dst, up)) {
-            best = g2;
-            dst = c2;
-        }
-    }
+    warp_argmax(best, dst, up);
     if constexpr (GT > 32) {
         // the group's warps are [w0, w0 + GT/32) of the block (several groups
         // may share a block)
@@ -553,8 +594,8 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
         if (A.agg) insert(rk, rs);  // every lane's last run
         // group totals of e and self weight, folded into the barrier that
         // publishes the table
-        e_part = warp_sum(e_part);
-        s_part = warp_sum(s_part);
+        e_part = value_sum(e_part);
+        s_part = value_sum(s_part);
         if ((threadIdx.x & 31) == 0) {
             if (e_part != V(0)) atomicAdd(&acc_e[par][g], e_part);
             if (s_part != V(0)) atomicAdd(&acc_s[par][g], s_part);
@@ -609,15 +650,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
         // warps' winners meet in shared memory behind one barrier and thread 0
         // of the group takes the best.  The table was cleaned during the
         // evaluation, before that barrier, so the next vertex may start.
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            G g2 = shfl_xor_g(best, o);
-            uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-            if (better(g2, c2, best, dst, up)) {
-                best = g2;
-                dst = c2;
-            }
-        }
+        warp_argmax(best, dst, up);
         if constexpr (GT > 32) {
             const int warp = threadIdx.x >> 5;
             if ((threadIdx.x & 31) == 0) {
@@ -808,7 +841,7 @@ __global__ void __launch_bounds__(kWarpThreads) lm_warp_kernel(LMArgs A, uint32_
                 }
                 // last step of vertex k: its internal and self weight
                 if (((f0 + 32) & (D - 1)) == 0) {
-                    const V te = warp_sum(e_part), ts = warp_sum(s_part);
+                    const V te = value_sum(e_part), ts = value_sum(s_part);
                     if (lane == 0) {
                         acc_e[k] += te;
                         acc_s[k] += ts;
@@ -865,15 +898,7 @@ __global__ void __launch_bounds__(kWarpThreads) lm_warp_kernel(LMArgs A, uint32_
                     }
                 }
                 if (((f0 + 32) & (D - 1)) == 0) {  // last step of vertex k: argmax, result
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const G g2 = shfl_xor_g(best, o);
-                        const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-                        if (better(g2, c2, best, dst, up)) {
-                            best = g2;
-                            dst = c2;
-                        }
-                    }
+                    warp_argmax(best, dst, up);
                     if (lane == k && act) {
                         vv.N[i] = final_choice<VER>(dst, src, up);
                         put_sin<BT>(A, i, sin, v2d(acc_e[k]) + v2d(acc_s[k]));
@@ -1615,16 +1640,9 @@ __global__ void __launch_bounds__(256) lm_first_kernel(LMArgs A, uint32_t bin_of
                 }
             }
         }
+        tile_argmax<T>(best, dst, up);
 #pragma unroll
-        for (int o = T / 2; o > 0; o >>= 1) {
-            const G g2 = shfl_xor_g(best, o);
-            const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-            if (better(g2, c2, best, dst, up)) {
-                best = g2;
-                dst = c2;
-            }
-            selfw += __shfl_xor_sync(0xffffffffu, selfw, o);
-        }
+        for (int o = T / 2; o > 0; o >>= 1) selfw += __shfl_xor_sync(0xffffffffu, selfw, o);
         if (active && gl == 0) {
             A.N[i] = final_choice<VER>(dst, i, up);
             sin += selfw;
@@ -1680,16 +1698,8 @@ __global__ void __launch_bounds__(BLOCK) lm_first_block_kernel(LMArgs A, uint32_
                 }
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const G g2 = shfl_xor_g(best, o);
-            const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-            if (better(g2, c2, best, dst, up)) {
-                best = g2;
-                dst = c2;
-            }
-            selfw += __shfl_xor_sync(0xffffffffu, selfw, o);
-        }
+        warp_argmax(best, dst, up);
+        selfw = warp_sum(selfw);
         if (lane == 0) {
             red_g[warp] = best;
             red_c[warp] = dst;

@@ -124,10 +124,15 @@ __device__ __forceinline__ void tile_task(const ResidentArgs &A, const uint32_t 
                 for (uint32_t mset = peers; mset; mset &= mset - 1) ks += sh.wbuf[warp][__ffs(mset) - 1];
             __syncwarp();
             V es = inner ? w[u] : V(0), ss = self ? w[u] : V(0);
+            if constexpr (T == 32) {
+                es = value_sum(es);
+                ss = value_sum(ss);
+            } else {
 #pragma unroll
-            for (int o = T / 2; o > 0; o >>= 1) {
-                es += __shfl_xor_sync(0xffffffffu, es, o);
-                ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                for (int o = T / 2; o > 0; o >>= 1) {
+                    es += __shfl_xor_sync(0xffffffffu, es, o);
+                    ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                }
             }
             kic = v2d(ks);
             e_src = v2d(es);
@@ -143,15 +148,7 @@ __device__ __forceinline__ void tile_task(const ResidentArgs &A, const uint32_t 
             }
             dcnt++;
         }
-#pragma unroll
-        for (int o = T / 2; o > 0; o >>= 1) {
-            const G g2 = shfl_xor_g(best, o);
-            const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-            if (better(g2, c2, best, dst, up)) {
-                best = g2;
-                dst = c2;
-            }
-        }
+        tile_argmax<T>(best, dst, up);
         if (act[u] && gl == 0) {
             N[i[u]] = final_choice<VER>(dst, src[u], up);
             sin += e_src + selfw;
@@ -249,8 +246,8 @@ __device__ __forceinline__ void hash_vertex(const ResidentArgs &A, const uint32_
         }
     }
     if (agg) insert(rk, rs);
-    e_part = warp_sum(e_part);
-    s_part = warp_sum(s_part);
+    e_part = value_sum(e_part);
+    s_part = value_sum(s_part);
     if constexpr (GT > 32) {
         if (lane == 0) {
             if (e_part != V(0)) atomicAdd(&sh.acc_e[par][g], e_part);
@@ -308,15 +305,7 @@ __device__ __forceinline__ void hash_vertex(const ResidentArgs &A, const uint32_
             }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const G g2 = shfl_xor_g(best, o);
-        const uint32_t c2 = __shfl_xor_sync(0xffffffffu, dst, o);
-        if (better(g2, c2, best, dst, up)) {
-            best = g2;
-            dst = c2;
-        }
-    }
+    warp_argmax(best, dst, up);
     if constexpr (GT > 32) {
         const int warp = threadIdx.x >> 5;
         if (lane == 0) {
