@@ -33,10 +33,18 @@
 // decisions and the sigma update; the decision kernel ends the loop when no
 // graph is active or the launch's sweep budget is used up, and the host
 // relaunches while graphs remain active.
+//
+// Where the graphs of a phase are small enough to be spread evenly, none of
+// this runs: the resident batch kernel (resident.cuh) takes every graph through
+// all its iterations with a cluster of CTAs (resident_phase below).
+#include <algorithm>
 #include <cmath>
+#include <cstddef>
+#include <cstring>
 #include <memory>
 
 #include "handles.cuh"
+#include "resident_args.cuh"
 
 namespace mg {
 
@@ -323,6 +331,9 @@ __global__ void list_scatter_kernel(const uint32_t *list, const uint32_t *lgid, 
     }
 }
 
+struct Idx19 {
+    uint32_t v[kSweepClasses + 1];
+};
 struct Idx12 {
     uint32_t v[kLightClasses + 1];
 };
@@ -467,6 +478,143 @@ void build_phase_graph(mg_ctx *ctx, mg_batch *b, const Body &B, cudaStream_t s, 
     MG_CUDA(cudaGraphInstantiate(&pg.exec, pg.graph, 0));
 }
 
+// ---- resident form: a graph per cluster of CTAs --------------------------------
+
+// start of every graph's part of every degree class: class lists are in id
+// order and a graph's vertices are consecutive ids
+__global__ void class_starts_kernel(const uint32_t *perm, Idx19 off, const uint32_t *goff, uint32_t G, uint32_t *out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (G + 1) * kSweepClasses) return;
+    const uint32_t g = i / kSweepClasses, c = i % kSweepClasses, v = goff[g];
+    uint32_t lo = off.v[c], hi = off.v[c + 1];
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (perm[mid] < v) lo = mid + 1;
+        else hi = mid;
+    }
+    out[i] = lo;
+}
+
+// CTAs per graph for a phase of the resident kernel, 0 when the class kernels
+// serve it better.  Both are estimated per sweep: a CTA sweeps kSmRate entries
+// per microsecond and a sweep takes kSweepMin at least; clusters take the graphs
+// in turn, largest first, so a phase ends after the mean load of a cluster plus
+// at most one graph.  The class kernels sweep kClassRate entries per microsecond
+// over all graphs and pay kClassSweep per sweep for launches and the per-graph
+// sums.  (One graph among many that is too large for a cluster, or a vertex
+// of more communities than a CTA's table holds, sends the phase there.)
+int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vector<uint32_t> &alive,
+                  const std::vector<uint64_t> &load, uint32_t most_vertices) {
+    constexpr double kSmRate = 365, kSweepMin = 8, kClassRate = 42e3, kClassSweep = 120;
+    if (ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
+    if (std::min(lvl.bins.max_degree, most_vertices) > lmr::kResidentCapacity) return 0;
+    double total = 0;
+    for (uint32_t g : alive) total += (double)load[g];
+    double best = total / kClassRate + kClassSweep;
+    int ctas = 0;
+    for (int cs = 1; cs <= 8; cs *= 2) {
+        double sum = 0, most = 0;
+        for (uint32_t g : alive) {
+            const double t = std::max(kSweepMin, (double)load[g] / (cs * kSmRate));
+            sum += t;
+            most = std::max(most, t);
+        }
+        const double clusters = kNumSMs / cs;
+        const double est = std::max(most, sum / clusters + most * (1 - 1 / clusters));
+        if (est < best) {
+            best = est;
+            ctas = cs;
+        }
+    }
+    return ctas;
+}
+
+void launch_batch(const lmr::ResidentBatchArgs &A, int wk, const SweepParams &p, int ctas, unsigned most,
+                  cudaStream_t s) {
+    if (wk == WK_UNIT) lmr::launch_batch_unit(A, p.precision, p.version, ctas, most, s);
+    else if (wk == WK_U32) lmr::launch_batch_u32(A, p.precision, p.version, ctas, most, s);
+    else if (wk == WK_F32I) lmr::launch_batch_f32i(A, p.precision, p.version, ctas, most, s);
+    else if (wk == WK_F64I) lmr::launch_batch_f64i(A, p.precision, p.version, ctas, most, s);
+    else if (wk == WK_F32) lmr::launch_batch_f32(A, p.precision, p.version, ctas, most, s);
+    else lmr::launch_batch_f64(A, p.precision, p.version, ctas, most, s);
+}
+
+// All iterations of the phase for the graphs `order` (largest first).  Leaves
+// what the iteration loop leaves: base buffers in the control words, Q and
+// iteration counts per graph.
+void resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLevel &lvl, const SweepParams &p,
+                    double thr, const uint32_t *goff, std::vector<uint32_t> order, int ctas, mg_summary &S,
+                    cudaStream_t s) {
+    using namespace lmr;
+    BatchWork &W = b->work;
+    const uint32_t G = b->graphs;
+    Idx19 off = {};
+    for (int c = 0; c < kSweepClasses; c++) off.v[c] = lvl.bins.offset[c];
+    off.v[kSweepClasses] = g.n;
+    uint32_t *cls = W.rcls.ensure((size_t)(G + 1) * kSweepClasses);
+    class_starts_kernel<<<(unsigned)ceil_div((uint64_t)(G + 1) * kSweepClasses, 256), 256, 0, s>>>(
+        ctx->mws.perm.get(), off, goff, G, cls);
+    MG_LAUNCH_CHECK();
+    struct Tail {
+        ResidentTotals totals;
+        uint32_t queue, pad;
+    };
+    unsigned char *mem = W.rstate.ensure(sizeof(ResidentState) * (size_t)G + sizeof(Tail));
+    ResidentState *state = (ResidentState *)mem;
+    Tail *tail = (Tail *)(mem + sizeof(ResidentState) * (size_t)G);
+    std::vector<ResidentState> hs(G);
+    memset(hs.data(), 0, sizeof(ResidentState) * G);
+    for (uint32_t q : order) {
+        hs[q].nx = 1;
+        hs[q].up = 1;
+        hs[q].first = 1;
+    }
+    MG_CUDA(cudaMemcpyAsync(state, hs.data(), sizeof(ResidentState) * G, cudaMemcpyHostToDevice, s));
+    uint32_t *d_order = W.rorder.ensure(G);
+    ResidentBatchArgs A = {};
+    A.col = g.col;
+    A.w = g.w;
+    A.perm = ctx->mws.perm.get();
+    A.rows = ctx->mws.rows.get();
+    A.k = ctx->k.get();
+    A.sigma = ctx->sigma.get();
+    for (int i = 0; i < 3; i++) A.C[i] = ctx->C[i].get();
+    A.thr = thr;
+    A.integral = p.integral;
+    A.bits = resident_bits(lvl.bins.max_degree);
+    A.cls = cls;
+    A.goff = goff;
+    A.gnnz = W.gnnz.get();
+    A.gk = W.gk.get();
+    A.mass = W.gmass.get();
+    A.order = d_order;
+    A.queue = &tail->queue;
+    A.state = state;
+    A.gword = W.gword.get();
+    A.curQ = W.curQ.get();
+    A.iters = W.iters.get();
+    A.distinct = &ctx->mws.acc.get()->distinct;
+    A.totals = &tail->totals;
+    const int wk = p.integral ? (g.wk == WK_F32 ? (int)WK_F32I : g.wk == WK_F64 ? (int)WK_F64I : g.wk) : g.wk;
+    unsigned long long sweeps = 0;
+    while (!order.empty()) {
+        A.count = (uint32_t)order.size();
+        MG_CUDA(cudaMemcpyAsync(d_order, order.data(), sizeof(uint32_t) * order.size(), cudaMemcpyHostToDevice, s));
+        MG_CUDA(cudaMemsetAsync(tail, 0, sizeof(Tail), s));
+        launch_batch(A, wk, p, ctas, A.count, s);
+        Tail ht;
+        MG_CUDA(cudaMemcpyAsync(&ht, tail, sizeof ht, cudaMemcpyDeviceToHost, s));
+        MG_CUDA(cudaStreamSynchronize(s));
+        S.edges_swept += ht.totals.edges;
+        sweeps = std::max(sweeps, ht.totals.sweeps);
+        if (!ht.totals.open) break;
+        MG_CUDA(cudaMemcpyAsync(hs.data(), state, sizeof(ResidentState) * G, cudaMemcpyDeviceToHost, s));
+        MG_CUDA(cudaStreamSynchronize(s));
+        order.erase(std::remove_if(order.begin(), order.end(), [&](uint32_t q) { return hs[q].done; }), order.end());
+    }
+    S.sweeps += sweeps;
+}
+
 }  // namespace
 
 void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &res, const GraphDoneFn *done) {
@@ -542,6 +690,9 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
     }
     if (n0 > 0) fill_identity(assign, n0, s);
     std::vector<uint32_t> hgoff(b->voff.begin(), b->voff.end()), hgoff_new(G + 1);
+    std::vector<uint32_t> hnnz(G);
+    std::vector<uint64_t> load(G);
+    for (uint32_t g = 0; g < G; g++) hnnz[g] = (uint32_t)(b->eoff[g + 1] - b->eoff[g]);
     std::vector<double> hq(G), Qh(G, 0.0), Qold(G, -1.0);
     std::vector<int> phases(G, 0);
     // results handed out early (done callback): graphs without edges now,
@@ -591,82 +742,100 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
                                                                      W.loops.get(), ctrl);
         MG_LAUNCH_CHECK();
         level_init(cur, k, sigma, C[0], s);
+        if (phase > 0)  // (level 0: the batch's own entry offsets)
+            MG_CUDA(cudaMemcpyAsync(hnnz.data(), W.gnnz.get(), sizeof(uint32_t) * G, cudaMemcpyDeviceToHost, s));
         move_prepare_level(cur, mlv, ctx->mws, s);
+        MG_CUDA(cudaStreamSynchronize(s));
         sweep_reset_acc(ctx->mws, s);
-        // active lists of the phase
-        Lists Ls;
-        rebuild_lists(ctx, W, mlv, Ls, true, n, s);
-        Body B;
-        B.g = &cur;
-        B.sp = sp;
-        B.bs.gid = gid;
-        B.bs.gword = W.gword.get();
-        B.bs.gk = gk;
-        B.bs.C[0] = C[0];
-        B.bs.C[1] = C[1];
-        B.bs.C[2] = C[2];
-        B.bs.sinv = W.sinv.get();
-        B.bs.up = &ctrl->up;
-        B.goff = goff;
-        B.G = G;
-        B.thr = thr;
-        B.k = k;
-        B.sigma = sigma;
-        auto use_lists = [&]() {
-            B.lvl = &Ls.lvl;
-            B.bs.perm = W.lperm[Ls.cur].get();
-            B.bs.pgid = W.lpgid[Ls.cur].get();
-            B.vlist = W.lvert[Ls.cur].get();
-            B.vgid = W.lvgid[Ls.cur].get();
-            B.vlen = Ls.vlen;
-            W.h_ctrl->listed = Ls.vlen;
-            MG_CUDA(cudaMemcpyAsync(&ctrl->listed, &W.h_ctrl->listed, sizeof(unsigned long long),
-                                    cudaMemcpyHostToDevice, s));
-        };
-        use_lists();
-        // shapes of the light classes (autotuner): the timing runs write what
-        // the first sweep of the phase writes
-        move_tune_batch(cur, Ls.lvl, ctx->mws, sp, B.bs, k, sigma, s);
-        // iterate until every graph has rejected a sweep.  The first sweep
-        // after the lists change runs as plain launches (it also sets up the
-        // launch shapes); the rest, with MG_BATCH_GRAPHS, as CUDA-graph loops.
-        std::unique_ptr<PhaseGraph> pg;
-        unsigned long long graph_sweeps0 = 0;
-        auto retire_graph = [&]() {
-            if (pg) g_kernel_launches += pg->body_launches * (W.h_ctrl->sweeps - graph_sweeps0);
-            pg.reset();
-        };
-        bool plain = true;
-        B.sp.agg = 0;  // the phase's first sweep: every community is one vertex
-        B.sp.split = sweep_split(ctx->mws, 0);
-        while (true) {
-            if (use_graph && !plain) {
-                if (!pg) {
-                    pg.reset(new PhaseGraph());
-                    build_phase_graph(ctx, b, B, s, *pg);
-                    graph_sweeps0 = W.h_ctrl->sweeps;
-                }
-                W.h_ctrl->budget = kGraphBudget;
-                MG_CUDA(cudaMemcpyAsync(&ctrl->budget, &W.h_ctrl->budget, sizeof(long long), cudaMemcpyHostToDevice,
-                                        s));
-                MG_CUDA(cudaGraphLaunch(pg->exec, s));
-            } else {
-                run_body(ctx, b, B, s, 0, cudaGraphConditionalHandle());
-            }
-            plain = false;
-            B.sp.agg = 1;  // later sweeps: communities repeat among neighbours
-            B.sp.split = sweep_split(ctx->mws, 1);
-            MG_CUDA(cudaMemcpyAsync(W.h_ctrl, ctrl, sizeof(BatchCtrl), cudaMemcpyDeviceToHost, s));
-            MG_CUDA(cudaStreamSynchronize(s));
-            if (W.h_ctrl->active == 0) break;
-            if (2 * W.h_ctrl->active_vertices <= W.h_ctrl->listed) {
-                retire_graph();
-                rebuild_lists(ctx, W, mlv, Ls, false, n, s);
-                use_lists();
-                plain = true;
-            }
+        std::vector<uint32_t> order;
+        uint32_t most_vertices = 0;
+        for (uint32_t g = 0; g < G; g++) {
+            if (!alive[g]) continue;
+            order.push_back(g);
+            const uint32_t ng = hgoff[g + 1] - hgoff[g];
+            most_vertices = std::max(most_vertices, ng);
+            load[g] = hnnz[g] + 4ull * ng;
         }
-        retire_graph();
+        const int ctas = resident_ctas(ctx->mws, mlv, order, load, most_vertices);
+        if (ctas > 0) {
+            std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return load[x] > load[y]; });
+            resident_phase(ctx, b, cur, mlv, sp, thr, goff, order, ctas, S, s);
+        } else {
+            // active lists of the phase
+            Lists Ls;
+            rebuild_lists(ctx, W, mlv, Ls, true, n, s);
+            Body B;
+            B.g = &cur;
+            B.sp = sp;
+            B.bs.gid = gid;
+            B.bs.gword = W.gword.get();
+            B.bs.gk = gk;
+            B.bs.C[0] = C[0];
+            B.bs.C[1] = C[1];
+            B.bs.C[2] = C[2];
+            B.bs.sinv = W.sinv.get();
+            B.bs.up = &ctrl->up;
+            B.goff = goff;
+            B.G = G;
+            B.thr = thr;
+            B.k = k;
+            B.sigma = sigma;
+            auto use_lists = [&]() {
+                B.lvl = &Ls.lvl;
+                B.bs.perm = W.lperm[Ls.cur].get();
+                B.bs.pgid = W.lpgid[Ls.cur].get();
+                B.vlist = W.lvert[Ls.cur].get();
+                B.vgid = W.lvgid[Ls.cur].get();
+                B.vlen = Ls.vlen;
+                W.h_ctrl->listed = Ls.vlen;
+                MG_CUDA(cudaMemcpyAsync(&ctrl->listed, &W.h_ctrl->listed, sizeof(unsigned long long),
+                                        cudaMemcpyHostToDevice, s));
+            };
+            use_lists();
+            // shapes of the light classes (autotuner): the timing runs write what
+            // the first sweep of the phase writes
+            move_tune_batch(cur, Ls.lvl, ctx->mws, sp, B.bs, k, sigma, s);
+            // iterate until every graph has rejected a sweep.  The first sweep
+            // after the lists change runs as plain launches (it also sets up the
+            // launch shapes); the rest, with MG_BATCH_GRAPHS, as CUDA-graph loops.
+            std::unique_ptr<PhaseGraph> pg;
+            unsigned long long graph_sweeps0 = 0;
+            auto retire_graph = [&]() {
+                if (pg) g_kernel_launches += pg->body_launches * (W.h_ctrl->sweeps - graph_sweeps0);
+                pg.reset();
+            };
+            bool plain = true;
+            B.sp.agg = 0;  // the phase's first sweep: every community is one vertex
+            B.sp.split = sweep_split(ctx->mws, 0);
+            while (true) {
+                if (use_graph && !plain) {
+                    if (!pg) {
+                        pg.reset(new PhaseGraph());
+                        build_phase_graph(ctx, b, B, s, *pg);
+                        graph_sweeps0 = W.h_ctrl->sweeps;
+                    }
+                    W.h_ctrl->budget = kGraphBudget;
+                    MG_CUDA(cudaMemcpyAsync(&ctrl->budget, &W.h_ctrl->budget, sizeof(long long), cudaMemcpyHostToDevice,
+                                            s));
+                    MG_CUDA(cudaGraphLaunch(pg->exec, s));
+                } else {
+                    run_body(ctx, b, B, s, 0, cudaGraphConditionalHandle());
+                }
+                plain = false;
+                B.sp.agg = 1;  // later sweeps: communities repeat among neighbours
+                B.sp.split = sweep_split(ctx->mws, 1);
+                MG_CUDA(cudaMemcpyAsync(W.h_ctrl, ctrl, sizeof(BatchCtrl), cudaMemcpyDeviceToHost, s));
+                MG_CUDA(cudaStreamSynchronize(s));
+                if (W.h_ctrl->active == 0) break;
+                if (2 * W.h_ctrl->active_vertices <= W.h_ctrl->listed) {
+                    retire_graph();
+                    rebuild_lists(ctx, W, mlv, Ls, false, n, s);
+                    use_lists();
+                    plain = true;
+                }
+            }
+            retire_graph();
+        }
         SweepAcc hacc;
         MG_CUDA(cudaMemcpyAsync(&hacc, ctx->mws.acc.get(), sizeof(SweepAcc), cudaMemcpyDeviceToHost, s));
         MG_CUDA(cudaMemcpyAsync(hq.data(), W.curQ.get(), sizeof(double) * G, cudaMemcpyDeviceToHost, s));
@@ -757,8 +926,8 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
     float ms = 0;
     MG_CUDA(cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]));
     S.seconds_total = ms * 1e-3;
-    S.sweeps = W.h_ctrl->sweeps;
-    S.edges_swept = W.h_ctrl->edges;
+    S.sweeps += W.h_ctrl->sweeps;  // (the resident phases have added theirs)
+    S.edges_swept += W.h_ctrl->edges;
     S.kernel_launches = g_kernel_launches - launches0;
     for (uint32_t g = 0; g < G; g++) {
         mg_batch_graph_summary &P = res.per[g];

@@ -103,6 +103,10 @@ struct BatchWork {
     DBuf<unsigned char> gen;
     DBuf<int> bad;
     DBuf<uint8_t> alive;
+    // resident batch kernel: class ranges and queue order of the graphs; their
+    // loop states, then totals and queue
+    DBuf<uint32_t> rcls, rorder;
+    DBuf<unsigned char> rstate;
     LevelGraph built;  // swapped with the union's buffers by the generator
     ~BatchWork();
 };

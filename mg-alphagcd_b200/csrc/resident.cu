@@ -24,7 +24,7 @@ struct ResidentBlock {
 }  // namespace
 
 bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws) {
-    if (ws.forced_policy || g.n == 0 || g.nnz > kResidentMaxEntries) return false;
+    if (ws.forced_policy || ws.tune.mode != MG_TUNE_ON || g.n == 0 || g.nnz > kResidentMaxEntries) return false;
     return std::min(lvl.bins.max_degree, g.n) <= kResidentCapacity;
 }
 
@@ -52,42 +52,14 @@ void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const S
     A.n = g.n;
     A.nnz = g.nnz;
     A.integral = p.integral;
-    // The table: as small as the level allows, since what it does not take
-    // stays L1 for the community and sigma gathers.
-    const uint32_t most = std::min(B.max_degree, g.n);
-    A.bits = most <= 32 ? 10 : most <= 64 ? 12 : most <= 128 ? 13 : kResidentMaxBits;
-    const uint32_t S = 1u << A.bits;
-    auto class_of = [](uint32_t deg) {  // last class of degrees <= deg (a power of two)
-        int c = 0;
-        while ((1u << c) < deg) c++;
-        return c;
-    };
-    const int cw = std::max(5, class_of(S / 64)), c128 = std::max(cw, class_of(S / 16)),
-              c256 = std::max(c128, class_of(S / 8));
-    auto start = [&](int c) { return c < kSweepClasses ? B.offset[c] : g.n; };
-    A.cut[1] = start(cw + 1);
-    A.cut[2] = start(c128 + 1);
-    A.cut[3] = start(c256 + 1);
-    A.cut[4] = g.n;
-    A.kind_off[0] = start(6);
-    A.kind_size[0] = A.cut[1] - start(6);
-    for (int kd = 1; kd <= 5; kd++) {
-        const int c = 6 - kd;  // classes 5, 4, 3, 2 and (one kind) 1 with 0
-        const uint32_t o = kd == 5 ? 0 : start(c);
-        A.kind_off[kd] = o;
-        A.kind_size[kd] = start(c + 1) - o;
-    }
-    uint32_t tasks = 0;
-    for (int kd = 0; kd < 6; kd++) {
-        const uint32_t per = kd == 0 ? 1 : kTileU << (kd - 1);
-        tasks += (uint32_t)ceil_div(A.kind_size[kd], per);
-        A.task_end[kd] = tasks;
-    }
-    A.tasks = tasks;
-    // CTAs: half a CTA's warps busy with a task each, or one per large vertex
-    const uint64_t want = ceil_div(tasks, kResidentThreads / 64) + (A.cut[2] - A.cut[1] + 7) / 8 +
-                          (A.cut[3] - A.cut[2] + 3) / 4 + (A.cut[4] - A.cut[3]);
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, kNumSMs));
+    A.bits = resident_bits(std::min(B.max_degree, g.n));
+    for (int c = 0; c < kSweepClasses; c++) A.cls[c] = B.offset[c];
+    A.cls[kSweepClasses] = g.n;
+    // CTAs: work for half of a CTA's warps, or as many as there are SMs
+    uint64_t warps = 0;
+    for (int c = 0; c < kSweepClasses; c++)
+        warps += c > 5 ? B.size[c] * ceil_div(1ull << c, 1ull << (A.bits - 6)) : ceil_div(B.size[c], kTileU * (32u >> c));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(warps, 16), kNumSMs));
     A.state = &db->state;
     A.acc = db->acc;
     A.task_ctr = db->task_ctr;

@@ -61,13 +61,43 @@ struct Shared {
     double red_sin[kWarps];
     unsigned long long red_d[kWarps], red_u[kWarps];
     double red_f[kWarps];
-    ResidentState st;  // the loop's state, the same in every CTA
+    ResidentState st;  // the loop's state, the same in every CTA of the team
     int ok;
+    // the graph's part of the class list: vertices [beg[c], end[c]) per degree
+    // class, and the warp tasks of classes cw .. 0, cumulative
+    uint32_t beg[kSweepClasses], end[kSweepClasses];
+    uint32_t task_end[kSweepClasses];
+    uint32_t chunk;  // tasks taken at a time
 };
 
+// Last classes whose vertices fit a warp's, 128 threads' and 256 threads' part
+// of a table of 2^bits slots (2 * degree slots); tiles serve classes 0-5.
+__device__ __forceinline__ int class_warp(int bits) { return max(5, bits - 6); }
+__device__ __forceinline__ int class_128(int bits) { return max(class_warp(bits), bits - 4); }
+__device__ __forceinline__ int class_256(int bits) { return max(class_warp(bits), bits - 3); }
+
+// Task counts of the warp stage from the class ranges (one thread), for a team
+// of `size` CTAs.  A warp takes up to 16 tasks with one atomic, an eighth of its
+// share: with one task each, the counter's address was the limit of a sweep
+// (1.5 atomics per ns; SBM of 4.0 M entries 60 us a sweep).
+template <class SH>
+__device__ __forceinline__ void count_tasks(SH &sh, int bits, uint32_t size) {
+    uint32_t sum = 0;
+    const int cw = class_warp(bits);
+    for (int i = 0; i <= cw; i++) {
+        const int c = cw - i;
+        const uint32_t m = sh.end[c] - sh.beg[c];
+        const uint32_t per = c > 5 ? 1u : kTileU << (c == 0 ? 4 : 5 - c);
+        sum += (m + per - 1) / per;
+        sh.task_end[i] = sum;
+    }
+    sh.chunk = max(1u, min(16u, sum / (size * kWarps * 8)));
+}
+
+
 // ---- degree <= 32: T lanes per vertex, U warp steps in flight ----------------
-template <int T, int U, int WK, int PREC, int VER, class SH>
-__device__ __forceinline__ void tile_task(const ResidentArgs &A, const uint32_t *P, uint32_t *N, uint32_t q0,
+template <int T, int U, int WK, int PREC, int VER, class AV, class SH>
+__device__ __forceinline__ void tile_task(const AV &A, const uint32_t *P, uint32_t *N, uint32_t q0,
                                           uint32_t q1, int up, double &sin, unsigned &dcnt, SH &sh) {
     using G = typename Prec<PREC>::G;
     using V = typename ValT<WK>::type;
@@ -158,8 +188,8 @@ __device__ __forceinline__ void tile_task(const ResidentArgs &A, const uint32_t 
 
 // ---- GT threads per vertex, shared-memory table of at most 2^bits slots ------
 // DENSE (the CTA's table): no insertion list, the evaluation scans the slots.
-template <int GT, int WK, int PREC, int VER, bool DENSE, class SH>
-__device__ __forceinline__ void hash_vertex(const ResidentArgs &A, const uint32_t *P, uint32_t *N, uint32_t q, int up,
+template <int GT, int WK, int PREC, int VER, bool DENSE, class AV, class SH>
+__device__ __forceinline__ void hash_vertex(const AV &A, const uint32_t *P, uint32_t *N, uint32_t q, int up,
                                             int agg, uint32_t *keys, typename ValT<WK>::type *vals, uint16_t *used,
                                             int max_bits, int &par, double &sin, unsigned &dcnt, SH &sh) {
     using G = typename Prec<PREC>::G;
@@ -353,6 +383,177 @@ __device__ __forceinline__ bool grid_wait(unsigned *ctr, unsigned target) {
     return false;
 }
 
+// The vertices of classes [c0, c1], largest first, that fall to group `x` of
+// `groups`; f(q) works entry q of the class list.
+template <class SH, class F>
+__device__ __forceinline__ void each_vertex(const SH &sh, int c0, int c1, uint32_t x, uint32_t groups, F f) {
+    for (int c = c1; c >= c0; c--) {
+        const uint32_t m = sh.end[c] - sh.beg[c];
+        for (; x < m; x += groups) f(sh.end[c] - 1 - x);
+        x -= m;
+    }
+}
+
+// One sweep of a graph by a team of CTAs (this one is `rank` of `size`): the
+// vertices of its class ranges, P -> N.  grab() hands out the next warp task.
+template <int WK, int PREC, int VER, class AV, class SH, class Grab>
+__device__ __forceinline__ void team_sweep(const AV &A, const uint32_t *P, uint32_t *N, int up, int agg, int bits,
+                                           uint32_t rank, uint32_t size, uint32_t *keys,
+                                           typename ValT<WK>::type *vals, uint16_t *used, double &sin, unsigned &dcnt,
+                                           SH &sh, Grab grab) {
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    const uint32_t S = 1u << bits;
+    const int cw = class_warp(bits), c128 = class_128(bits), c256 = class_256(bits);
+    int par = 0;
+    // the CTA per vertex
+    each_vertex(sh, c256 + 1, kSweepClasses - 1, rank, size, [&](uint32_t q) {
+        hash_vertex<kThreads, WK, PREC, VER, true>(A, P, N, q, up, agg, keys, vals, used, bits, par, sin, dcnt, sh);
+    });
+    __syncthreads();  // the groups below reuse the sums of group 0
+    {
+        const uint32_t g = t / 256, sl = S / 4 * g;
+        par = 0;
+        each_vertex(sh, c128 + 1, c256, rank * 4 + g, size * 4, [&](uint32_t q) {
+            hash_vertex<256, WK, PREC, VER, false>(A, P, N, q, up, agg, keys + sl, vals + sl, used + sl / 2, bits - 2,
+                                                   par, sin, dcnt, sh);
+        });
+    }
+    __syncthreads();
+    {
+        const uint32_t g = t / 128, sl = S / 8 * g;
+        par = 0;
+        each_vertex(sh, cw + 1, c128, rank * 8 + g, size * 8, [&](uint32_t q) {
+            hash_vertex<128, WK, PREC, VER, false>(A, P, N, q, up, agg, keys + sl, vals + sl, used + sl / 2, bits - 3,
+                                                   par, sin, dcnt, sh);
+        });
+    }
+    // warp vertices and tiles, by task
+    const uint32_t sl = S / 32 * warp, tasks = sh.task_end[cw];
+    const uint32_t ch = sh.chunk;
+    uint32_t k = rank * kWarps + warp;  // chunk of tasks
+    while (k * ch < tasks) {
+        uint32_t nxt = 0;
+        if (lane == 0) nxt = size * kWarps + grab();
+        const uint32_t t1 = min(tasks, (k + 1) * ch);
+        for (uint32_t task = k * ch; task < t1; task++) {
+            int i = 0;
+            while (task >= sh.task_end[i]) i++;
+            const int c = cw - i;
+            const uint32_t k0 = task - (i ? sh.task_end[i - 1] : 0u);
+            const uint32_t q0 = sh.beg[c], q1 = sh.end[c];
+            if (c > 5)
+                hash_vertex<32, WK, PREC, VER, false>(A, P, N, q1 - 1 - k0, up, agg, keys + sl, vals + sl,
+                                                      used + sl / 2, bits - 5, par, sin, dcnt, sh);
+            else if (c == 5)
+                tile_task<32, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * kTileU, q1, up, sin, dcnt, sh);
+            else if (c == 4)
+                tile_task<16, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 2 * kTileU, q1, up, sin, dcnt, sh);
+            else if (c == 3)
+                tile_task<8, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 4 * kTileU, q1, up, sin, dcnt, sh);
+            else if (c == 2)
+                tile_task<4, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 8 * kTileU, q1, up, sin, dcnt, sh);
+            else
+                tile_task<2, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 16 * kTileU, q1, up, sin, dcnt, sh);
+        }
+        k = __shfl_sync(0xffffffffu, nxt, 0);
+    }
+}
+
+// sum of sigma^2 over the communities [c0, c1), a thread's part
+__device__ __forceinline__ void sigma_sq(const double *sigma, uint32_t c0, uint32_t c1, uint32_t step, int integral,
+                                         unsigned long long &su, double &sf) {
+    for (uint64_t c = c0; c < c1; c += step) {
+        const double s = sigma[c];
+        if (integral) {
+            const unsigned long long u = (unsigned long long)s;
+            su += u * u;
+        } else {
+            sf += s * s;
+        }
+    }
+}
+
+// A thread's parts of a sweep's sums, added up over the CTA: valid in thread 0.
+struct SweepSums {
+    double sin;
+    unsigned long long distinct, s2_u;
+    double s2_f;
+};
+template <class SH>
+__device__ __forceinline__ SweepSums cta_sums(double sin, unsigned dcnt, unsigned long long su, double sf, SH &sh) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    sin = warp_sum(sin);
+    const unsigned long long dw = warp_sum((unsigned long long)dcnt);
+    su = warp_sum(su);
+    sf = warp_sum(sf);
+    if (lane == 0) {
+        sh.red_sin[warp] = sin;
+        sh.red_d[warp] = dw;
+        sh.red_u[warp] = su;
+        sh.red_f[warp] = sf;
+    }
+    __syncthreads();
+    SweepSums r = {0, 0, 0, 0};
+    if (warp == 0) {
+        r.sin = warp_sum(sh.red_sin[lane]);
+        r.distinct = warp_sum(sh.red_d[lane]);
+        r.s2_u = warp_sum(sh.red_u[lane]);
+        r.s2_f = warp_sum(sh.red_f[lane]);
+    }
+    return r;
+}
+
+// Q of a sweep's input assignment, the host's operations each rounded as written
+__device__ __forceinline__ double sweep_q(double sin, double s2, double mass) {
+    return __dsub_rn(__ddiv_rn(sin, mass), __ddiv_rn(s2, __dmul_rn(mass, mass)));
+}
+
+// The accept / reject step after a sweep with Q(P) = Q.
+__device__ __forceinline__ void next_state(ResidentState &st, double Q, unsigned long long distinct, double thr) {
+    st.distinct = distinct;
+    st.iters++;
+    if (st.first || __dsub_rn(Q, st.curQ) > thr) {
+        // the move P -> N is taken; N is swept next
+        const int after = 3 - st.p - st.nx;
+        st.curQ = Q;
+        st.base = st.p;
+        st.p = st.nx;
+        st.nx = after;
+        st.up ^= 1;
+        st.first = 0;
+    } else {
+        st.done = 1;
+    }
+}
+
+// sigma follows the move P -> N of the vertices [v0, v1)
+template <class AV>
+__device__ __forceinline__ void move_sigma(const AV &A, const uint32_t *P, const uint32_t *N, uint32_t v0, uint32_t v1,
+                                           uint32_t step) {
+    for (uint64_t v = v0; v < v1; v += step) {
+        const uint32_t x = P[v], y = N[v];
+        if (x != y) {
+            const double kv = A.k[v];
+            atomicAdd(A.sigma + x, -kv);
+            atomicAdd(A.sigma + y, kv);
+        }
+    }
+}
+
+// empty table, zero sums
+template <class V, class SH>
+__device__ __forceinline__ void clear_tables(uint32_t *keys, V *vals, uint32_t S, SH &sh) {
+    for (uint32_t s = threadIdx.x; s < S; s += kThreads) {
+        keys[s] = kEmpty;
+        vals[s] = V(0);
+    }
+    if (threadIdx.x < 16) {
+        (&sh.cnt[0][0])[threadIdx.x] = 0;
+        (&sh.acc_e[0][0])[threadIdx.x] = V(0);
+        (&sh.acc_s[0][0])[threadIdx.x] = V(0);
+    }
+}
+
 template <int WK, int PREC, int VER>
 __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A) {
     using G = typename Prec<PREC>::G;
@@ -363,141 +564,46 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A
     V *vals = (V *)smem_raw;
     uint32_t *keys = (uint32_t *)(smem_raw + sizeof(V) * S);
     uint16_t *used = (uint16_t *)(smem_raw + (sizeof(V) + sizeof(uint32_t)) * S);
-    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    for (uint32_t s = t; s < S; s += kThreads) {
-        keys[s] = kEmpty;
-        vals[s] = V(0);
-    }
-    if (t < 16) {
-        (&sh.cnt[0][0])[t] = 0;
-        (&sh.acc_e[0][0])[t] = V(0);
-        (&sh.acc_s[0][0])[t] = V(0);
+    const uint32_t t = threadIdx.x;
+    clear_tables(keys, vals, S, sh);
+    if (t < kSweepClasses) {
+        sh.beg[t] = A.cls[t];
+        sh.end[t] = A.cls[t + 1];
     }
     if (t == 0) sh.st = *A.state;
     __syncthreads();
-    unsigned bar = 0;  // barriers passed
+    if (t == 0) count_tasks(sh, A.bits, gridDim.x);
+    __syncthreads();
+    unsigned bar = 0;  // barriers passed (thread 0)
     const uint32_t gthreads = gridDim.x * kThreads, gt = blockIdx.x * kThreads + t;
-    const uint32_t gwarps = gridDim.x * kWarps;
     for (int it = 0; it < kResidentIters; it++) {
         SweepAcc *acc = A.acc + it;
         const uint32_t *P = A.C[sh.st.p];
         uint32_t *N = A.C[sh.st.nx];
-        const int up = sh.st.up;
-        const int agg = !sh.st.first && 2 * sh.st.distinct < A.nnz;
-        double sin = 0;
+        double sin = 0, sf = 0;
         unsigned dcnt = 0;
-        int par = 0;
-        // the CTA per vertex, largest degrees first
-        for (uint32_t q = A.cut[3] + blockIdx.x; q < A.cut[4]; q += gridDim.x)
-            hash_vertex<kThreads, WK, PREC, VER, true>(A, P, N, A.cut[4] - 1 - (q - A.cut[3]), up, agg, keys, vals,
-                                                       used, A.bits, par, sin, dcnt, sh);
-        __syncthreads();  // the groups below reuse the sums of group 0
-        {
-            const uint32_t g = t / 256;
-            const uint32_t sl = S / 4 * g;
-            par = 0;
-            for (uint32_t q = A.cut[2] + blockIdx.x * 4 + g; q < A.cut[3]; q += gridDim.x * 4)
-                hash_vertex<256, WK, PREC, VER, false>(A, P, N, A.cut[3] - 1 - (q - A.cut[2]), up, agg, keys + sl,
-                                                       vals + sl, used + sl / 2, A.bits - 2, par, sin, dcnt, sh);
-        }
-        __syncthreads();
-        {
-            const uint32_t g = t / 128;
-            const uint32_t sl = S / 8 * g;
-            par = 0;
-            for (uint32_t q = A.cut[1] + blockIdx.x * 8 + g; q < A.cut[2]; q += gridDim.x * 8)
-                hash_vertex<128, WK, PREC, VER, false>(A, P, N, A.cut[2] - 1 - (q - A.cut[1]), up, agg, keys + sl,
-                                                       vals + sl, used + sl / 2, A.bits - 3, par, sin, dcnt, sh);
-        }
-        // warp vertices and tiles, by task
-        {
-            const uint32_t sl = S / 32 * warp;
-            uint32_t task = blockIdx.x * kWarps + warp;
-            while (task < A.tasks) {
-                uint32_t nxt = 0;
-                if (lane == 0) nxt = gwarps + atomicAdd(A.task_ctr + it, 1u);
-                int kind = 0;  // 0: warp vertices, 1..5: tiles of 32, 16, 8, 4, 2 lanes
-                while (kind < 5 && task >= A.task_end[kind]) kind++;
-                const uint32_t k0 = task - (kind ? A.task_end[kind - 1] : 0u);
-                const uint32_t q0 = A.kind_off[kind], q1 = A.kind_off[kind] + A.kind_size[kind];
-                if (kind == 0)
-                    hash_vertex<32, WK, PREC, VER, false>(A, P, N, q1 - 1 - k0, up, agg, keys + sl, vals + sl,
-                                                          used + sl / 2, A.bits - 5, par, sin, dcnt, sh);
-                else if (kind == 1)
-                    tile_task<32, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * kTileU, q1, up, sin, dcnt, sh);
-                else if (kind == 2)
-                    tile_task<16, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 2 * kTileU, q1, up, sin, dcnt, sh);
-                else if (kind == 3)
-                    tile_task<8, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 4 * kTileU, q1, up, sin, dcnt, sh);
-                else if (kind == 4)
-                    tile_task<4, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 8 * kTileU, q1, up, sin, dcnt, sh);
-                else
-                    tile_task<2, kTileU, WK, PREC, VER>(A, P, N, q0 + k0 * 16 * kTileU, q1, up, sin, dcnt, sh);
-                task = __shfl_sync(0xffffffffu, nxt, 0);
-            }
-        }
-        // sum of sigma^2 of P's communities
         unsigned long long su = 0;
-        double sf = 0;
-        for (uint32_t c = gt; c < A.n; c += gthreads) {
-            const double s = A.sigma[c];
+        team_sweep<WK, PREC, VER>(A, P, N, sh.st.up, !sh.st.first && 2 * sh.st.distinct < A.nnz, A.bits, blockIdx.x,
+                                  gridDim.x, keys, vals, used, sin, dcnt, sh,
+                                  [&] { return atomicAdd(A.task_ctr + it, 1u); });
+        sigma_sq(A.sigma, gt, A.n, gthreads, A.integral, su, sf);
+        const SweepSums r = cta_sums(sin, dcnt, su, sf, sh);
+        if (t == 0) {
             if (A.integral) {
-                const unsigned long long u = (unsigned long long)s;
-                su += u * u;
+                if (r.sin != 0) atomicAdd(&acc->sin_u, (unsigned long long)r.sin);
+                if (r.s2_u) atomicAdd(&acc->s2_u, r.s2_u);
             } else {
-                sf += s * s;
+                if (r.sin != 0) atomicAdd(&acc->sin_f, r.sin);
+                if (r.s2_f != 0) atomicAdd(&acc->s2_f, r.s2_f);
             }
-        }
-        sin = warp_sum(sin);
-        const unsigned long long dw = warp_sum((unsigned long long)dcnt);
-        su = warp_sum(su);
-        sf = warp_sum(sf);
-        if (lane == 0) {
-            sh.red_sin[warp] = sin;
-            sh.red_d[warp] = dw;
-            sh.red_u[warp] = su;
-            sh.red_f[warp] = sf;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            const double bs = warp_sum(lane < kWarps ? sh.red_sin[lane] : 0.0);
-            const unsigned long long bd = warp_sum(lane < kWarps ? sh.red_d[lane] : 0ull);
-            const unsigned long long bu = warp_sum(lane < kWarps ? sh.red_u[lane] : 0ull);
-            const double bf = warp_sum(lane < kWarps ? sh.red_f[lane] : 0.0);
-            if (lane == 0) {
-                if (A.integral) {
-                    if (bs != 0) atomicAdd(&acc->sin_u, (unsigned long long)bs);
-                    if (bu) atomicAdd(&acc->s2_u, bu);
-                } else {
-                    if (bs != 0) atomicAdd(&acc->sin_f, bs);
-                    if (bf != 0) atomicAdd(&acc->s2_f, bf);
-                }
-                if (bd) atomicAdd(&acc->distinct, bd);
-                bar++;
-                const bool ok = grid_wait(A.barrier, bar * gridDim.x);
-                sh.ok = ok;
-                // Q(P), the host's operations each rounded as written
-                const double x = A.integral ? __ull2double_rn(__ldcg(&acc->sin_u)) : __ldcg(&acc->sin_f);
-                const double y = A.integral ? __ull2double_rn(__ldcg(&acc->s2_u)) : __ldcg(&acc->s2_f);
-                const double Q = __dsub_rn(__ddiv_rn(x, A.mass), __ddiv_rn(y, __dmul_rn(A.mass, A.mass)));
-                if (blockIdx.x == 0) acc->pad = Q;
-                ResidentState st = sh.st;
-                st.distinct = __ldcg(&acc->distinct);
-                st.iters++;
-                if (st.first || __dsub_rn(Q, st.curQ) > A.thr) {
-                    // the move P -> N is taken; N is swept next
-                    const int after = 3 - st.p - st.nx;
-                    st.curQ = Q;
-                    st.base = st.p;
-                    st.p = st.nx;
-                    st.nx = after;
-                    st.up ^= 1;
-                    st.first = 0;
-                } else {
-                    st.done = 1;
-                }
-                sh.st = st;
-            }
+            if (r.distinct) atomicAdd(&acc->distinct, r.distinct);
+            bar++;
+            sh.ok = grid_wait(A.barrier, bar * gridDim.x);
+            const double x = A.integral ? __ull2double_rn(__ldcg(&acc->sin_u)) : __ldcg(&acc->sin_f);
+            const double y = A.integral ? __ull2double_rn(__ldcg(&acc->s2_u)) : __ldcg(&acc->s2_f);
+            const double Q = sweep_q(x, y, A.mass);
+            if (blockIdx.x == 0) acc->pad = Q;
+            next_state(sh.st, Q, __ldcg(&acc->distinct), A.thr);
         }
         __syncthreads();
         if (!sh.ok) {
@@ -505,14 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A
             return;
         }
         if (sh.st.done) break;
-        for (uint32_t v = gt; v < A.n; v += gthreads) {
-            const uint32_t x = P[v], y = N[v];
-            if (x != y) {
-                const double kv = A.k[v];
-                atomicAdd(A.sigma + x, -kv);
-                atomicAdd(A.sigma + y, kv);
-            }
-        }
+        move_sigma(A, P, N, gt, A.n, gthreads);
         __syncthreads();
         if (t == 0) {
             bar++;
@@ -526,6 +625,118 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A
     }
     // every CTA holds the same state; all read theirs before the first barrier
     if (blockIdx.x == 0 && t == 0) *A.state = sh.st;
+}
+
+// Many graphs packed as one union: a cluster of CTAs takes a graph through all
+// iterations of its phase, then the next one from the queue (largest first).
+// Graphs share nothing, so the clusters never wait for one another: the
+// barriers of an iteration are cluster barriers, the sums of a sweep are read
+// from the cluster's CTAs through distributed shared memory.
+template <int WK, int PREC, int VER>
+__global__ void __launch_bounds__(kThreads, 1) lm_resident_batch_kernel(ResidentBatchArgs A) {
+    using G = typename Prec<PREC>::G;
+    using V = typename ValT<WK>::type;
+    namespace cg = cooperative_groups;
+    struct View {
+        const uint32_t *col;
+        const void *w;
+        const uint32_t *perm;
+        const uint2 *rows;
+        const double *k;
+        double *sigma;
+        const GainK &K;
+    };
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ Shared<V, G> sh;
+    __shared__ GainK gk;
+    __shared__ SweepSums part[2];   // this CTA's sums, by the parity of the sweep
+    __shared__ uint32_t ctr[2];     // warp tasks handed out (rank 0's is the cluster's)
+    __shared__ uint32_t next, v0, v1;
+    __shared__ unsigned long long nnz;
+    __shared__ double mass;
+    cg::cluster_group cl = cg::this_cluster();
+    const uint32_t rank = cl.block_rank(), size = cl.num_blocks();
+    const uint32_t S = 1u << A.bits;
+    V *vals = (V *)smem_raw;
+    uint32_t *keys = (uint32_t *)(smem_raw + sizeof(V) * S);
+    uint16_t *used = (uint16_t *)(smem_raw + (sizeof(V) + sizeof(uint32_t)) * S);
+    const uint32_t t = threadIdx.x, lane = t & 31u;
+    const uint32_t tt = rank * kThreads + t, tn = size * kThreads;
+    clear_tables(keys, vals, S, sh);
+    if (t < 2) ctr[t] = 0;
+    const View view = {A.col, A.w, A.perm, A.rows, A.k, A.sigma, gk};
+    uint32_t *const ctr0 = cl.map_shared_rank(&ctr[0], 0);
+    while (true) {
+        if (rank == 0 && t == 0) next = atomicAdd(A.queue, 1u);
+        cl.sync();
+        const uint32_t qi = *cl.map_shared_rank(&next, 0);
+        if (qi >= A.count) break;
+        const uint32_t g = A.order[qi];
+        if (t < kSweepClasses) {
+            sh.beg[t] = A.cls[(size_t)g * kSweepClasses + t];
+            sh.end[t] = A.cls[(size_t)(g + 1) * kSweepClasses + t];
+        }
+        if (t == 0) {
+            gk = A.gk[g];
+            mass = A.mass[g];
+            nnz = A.gnnz[g];
+            v0 = A.goff[g];
+            v1 = A.goff[g + 1];
+            sh.st = A.state[g];
+        }
+        __syncthreads();
+        if (t == 0) count_tasks(sh, A.bits, size);
+        __syncthreads();
+        // (iterations of a launch are bounded; the host launches again)
+        for (int it = 0; it < kResidentBatchIters && !sh.st.done; it++) {
+            const int par = it & 1;
+            const uint32_t *P = A.C[sh.st.p];
+            uint32_t *N = A.C[sh.st.nx];
+            double sin = 0, sf = 0;
+            unsigned dcnt = 0;
+            unsigned long long su = 0;
+            team_sweep<WK, PREC, VER>(view, P, N, sh.st.up, !sh.st.first && 2 * sh.st.distinct < nnz, A.bits, rank,
+                                      size, keys, vals, used, sin, dcnt, sh,
+                                      [&] { return atomicAdd(ctr0 + par, 1u); });
+            sigma_sq(A.sigma, v0 + tt, v1, tn, A.integral, su, sf);
+            const SweepSums r = cta_sums(sin, dcnt, su, sf, sh);
+            if (t == 0) part[par] = r;
+            cl.sync();  // every CTA's sums, and the new assignment, are there
+            if (t < 32) {
+                SweepSums x = {0, 0, 0, 0};
+                if (lane < size) x = *cl.map_shared_rank(&part[par], lane);
+                x.sin = warp_sum(x.sin);
+                x.distinct = warp_sum(x.distinct);
+                x.s2_u = warp_sum(x.s2_u);
+                x.s2_f = warp_sum(x.s2_f);
+                if (lane == 0) {
+                    const double a = A.integral ? __ull2double_rn((unsigned long long)x.sin) : x.sin;
+                    const double b = A.integral ? __ull2double_rn(x.s2_u) : x.s2_f;
+                    next_state(sh.st, sweep_q(a, b, mass), x.distinct, A.thr);
+                    if (rank == 0) {
+                        ctr[par] = 0;  // every CTA is past this sweep's tasks
+                        atomicAdd(A.distinct, x.distinct);
+                    }
+                }
+            }
+            __syncthreads();
+            if (!sh.st.done) move_sigma(view, P, N, v0 + tt, v1, tn);
+            cl.sync();
+        }
+        if (rank == 0 && t == 0) {
+            A.state[g] = sh.st;
+            if (sh.st.done) {
+                A.gword[g] = gw_make(false, sh.st.p, sh.st.nx, sh.st.base, false, false, 0, 0);
+                A.curQ[g] = sh.st.curQ;
+                A.iters[g] += (unsigned long long)(sh.st.iters - 1);
+                atomicAdd(&A.totals->edges, nnz * (unsigned long long)sh.st.iters);
+                atomicMax(&A.totals->sweeps, (unsigned long long)sh.st.iters);
+            } else {
+                atomicAdd(&A.totals->open, 1u);
+            }
+        }
+    }
+    cl.sync();  // no CTA leaves while others may still read its memory
 }
 
 template <int WK>
@@ -549,6 +760,62 @@ void launch_resident(const ResidentArgs &A, unsigned grid, cudaStream_t s) {
     cfg.numAttrs = 1;
     MG_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
     MG_LAUNCH_CHECK();
+}
+
+template <int WK, int PREC, int VER>
+cudaLaunchConfig_t batch_config(const ResidentBatchArgs &A, int ctas, unsigned grid, cudaStream_t s,
+                                cudaLaunchAttribute *at) {
+    raise_smem_limit((const void *)lm_resident_batch_kernel<WK, PREC, VER>, resident_smem<WK>(kResidentMaxBits));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = resident_smem<WK>(A.bits);
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// As many clusters of `ctas` CTAs as the device holds, at most `most`.
+template <int WK, int PREC, int VER>
+void launch_batch(const ResidentBatchArgs &A, int ctas, unsigned most, cudaStream_t s) {
+    auto kern = lm_resident_batch_kernel<WK, PREC, VER>;
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = batch_config<WK, PREC, VER>(A, ctas, (unsigned)ctas, s, at);
+    int fit = 0;
+    MG_CUDA(cudaOccupancyMaxActiveClusters(&fit, (void *)kern, &cfg));
+    MG_CHECK(fit > 0, MG_ERR_UNSUPPORTED, "cluster shape cannot be scheduled on this device");
+    cfg.gridDim = dim3(std::min((unsigned)fit, most) * (unsigned)ctas);
+    MG_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+    MG_LAUNCH_CHECK();
+}
+
+template <int WK>
+void launch_batch_kind(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
+    auto version = [&](auto precc) {
+        constexpr int PREC = decltype(precc)::value;
+        if (ver == 1) launch_batch<WK, PREC, 1>(A, ctas, most, s);
+        else launch_batch<WK, PREC, 2>(A, ctas, most, s);
+    };
+    if (prec == MG_PREC_FP64) {
+        version(std::integral_constant<int, MG_PREC_FP64>());
+        return;
+    }
+    if (prec == MG_PREC_FP32) {
+        version(std::integral_constant<int, MG_PREC_FP32>());
+        return;
+    }
+    if constexpr (kIntg<WK>) {
+        if (prec == MG_PREC_INT64) {
+            version(std::integral_constant<int, MG_PREC_INT64>());
+            return;
+        }
+    }
+    throw Error(MG_ERR_INVALID, "unknown weight kind or precision");
 }
 
 template <int WK>

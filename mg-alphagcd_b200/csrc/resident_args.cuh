@@ -17,6 +17,13 @@ constexpr int kTileU = 2;
 // largest number of distinct communities a vertex may see: 2/3 of the CTA's table
 constexpr uint32_t kResidentCapacity = (1u << kResidentMaxBits) / 3 * 2;
 
+// log2 of the slots of a CTA's table for a level of that largest degree (or
+// number of communities a vertex can see): as small as the level allows, since
+// what the table does not take stays L1 for the community and sigma gathers
+inline int resident_bits(uint32_t most) {
+    return most <= 32 ? 10 : most <= 64 ? 12 : most <= 128 ? 13 : kResidentMaxBits;
+}
+
 // The loop's state, kept between launches: the assignment buffers (base: last
 // accepted, p: swept next, nx: written next), the direction, Q of the base.
 struct ResidentState {
@@ -39,17 +46,50 @@ struct ResidentArgs {
     unsigned long long nnz;
     int integral;
     int bits;  // log2 of the CTA's table slots
-    // class-list ranges: [cut[1], cut[2]) 128 threads per vertex, [cut[2],
-    // cut[3]) 256, [cut[3], cut[4]) the CTA
-    uint32_t cut[5];
-    // tasks of a warp: kind 0 a warp vertex, kinds 1..5 tiles of 32, 16, 8, 4
-    // and 2 lanes (kTileU steps each); task_end is cumulative
-    uint32_t kind_off[6], kind_size[6], task_end[6], tasks;
+    uint32_t cls[kSweepClasses + 1];  // start of every degree class in the class list; n
     ResidentState *state;
     SweepAcc *acc;       // one per iteration, zeroed; pad receives Q
     uint32_t *task_ctr;  // one per iteration, zeroed
     unsigned *barrier;   // zeroed
 };
+
+// The batched form (lm_resident_batch_kernel): a graph per cluster of CTAs.
+constexpr int kResidentBatchIters = 1024;  // iterations of a graph in one launch
+struct ResidentTotals {
+    unsigned long long edges;   // entries swept by the graphs that finished
+    unsigned long long sweeps;  // most sweeps of one graph
+    uint32_t open, pad;         // graphs that need another launch
+};
+struct ResidentBatchArgs {
+    const uint32_t *col;
+    const void *w;
+    const uint32_t *perm;
+    const uint2 *rows;
+    const double *k;
+    double *sigma;
+    uint32_t *C[3];
+    double thr;
+    int integral, bits;
+    const uint32_t *cls;    // per graph: start of its part of every degree class (graphs + 1 rows)
+    const uint32_t *goff;   // first vertex of each graph
+    const uint32_t *gnnz;
+    const GainK *gk;
+    const double *mass;
+    const uint32_t *order;  // graphs to run, largest first
+    uint32_t count;
+    uint32_t *queue;        // zeroed
+    ResidentState *state;   // per graph
+    uint32_t *gword;
+    double *curQ;
+    unsigned long long *iters, *distinct;
+    ResidentTotals *totals;  // zeroed
+};
+
+#define MG_RESIDENT_KINDS(X) X(unit) X(u32) X(f32i) X(f64i) X(f32) X(f64)
+#define MG_RESIDENT_BATCH(k) \
+    void launch_batch_##k(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s);
+MG_RESIDENT_KINDS(MG_RESIDENT_BATCH)
+#undef MG_RESIDENT_BATCH
 
 void launch_resident_unit(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
 void launch_resident_u32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);

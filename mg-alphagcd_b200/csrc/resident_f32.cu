@@ -1,4 +1,4 @@
-// resident_f32.cu -- the resident level kernel for weight kind WK_F32.
+// resident_f32.cu -- the resident level kernels for weight kind WK_F32.
 #include "resident.cuh"
 
 namespace mg {
@@ -6,6 +6,10 @@ namespace lmr {
 
 void launch_resident_f32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
     launch_resident_kind<WK_F32>(A, prec, ver, grid, s);
+}
+
+void launch_batch_f32(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
+    launch_batch_kind<WK_F32>(A, prec, ver, ctas, most, s);
 }
 
 }  // namespace lmr

@@ -1,4 +1,4 @@
-// resident_unit.cu -- the resident level kernel for weight kind WK_UNIT.
+// resident_unit.cu -- the resident level kernels for weight kind WK_UNIT.
 #include "resident.cuh"
 
 namespace mg {
@@ -6,6 +6,10 @@ namespace lmr {
 
 void launch_resident_unit(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
     launch_resident_kind<WK_UNIT>(A, prec, ver, grid, s);
+}
+
+void launch_batch_unit(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
+    launch_batch_kind<WK_UNIT>(A, prec, ver, ctas, most, s);
 }
 
 }  // namespace lmr
