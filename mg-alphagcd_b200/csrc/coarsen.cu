@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "tile_rows.cuh"
 
 namespace mg {
 
@@ -33,12 +34,8 @@ __global__ void apply_relabel_kernel(const uint32_t *C, uint32_t n, const uint32
 }
 
 // key = (C'[u] << bc) | C'[v] per edge (u,v), payload = weight (if any).
-// A block takes a tile of kExpandTile consecutive edges.  The rows that start
-// inside the tile are marked at their first edge (a row id per position; of
-// several rows starting at one position -- empty rows -- the largest, which is
-// the non-empty one, wins), a prefix maximum over the tile then gives every
-// edge its row, and the keys are written with coalesced loads and stores.
-// One binary search per tile finds the row holding its first edge.
+// A block takes a tile of kExpandTile consecutive edges, whose rows come from
+// tile_rows; the keys are written with coalesced loads and stores.
 // TR (symmetric graphs): the rows are visited in member order -- off holds
 // the offsets of the member-ordered expansion, member r's row starts at
 // msrc[r] of the graph and its community is mcom[r] (non-decreasing in r) --
@@ -52,27 +49,20 @@ __global__ void apply_relabel_kernel(const uint32_t *C, uint32_t n, const uint32
 // Pays where communities repeat within rows (the end of a phase whose last
 // sweep saw few distinct neighbour communities): the sort then sees far
 // fewer keys.
-constexpr int kExpandThreads = 256;
-constexpr int kExpandPer = 16;
-constexpr uint32_t kExpandTile = kExpandThreads * kExpandPer;
-
 template <int WK, class PV, bool COMBINE = false, bool TR = false>
 __global__ void __launch_bounds__(kExpandThreads)
     expand_keys_kernel(const uint32_t *off, const uint32_t *col, const void *w, uint32_t n, uint64_t m,
                        const uint32_t *Cd, int bc, uint64_t *keys, PV *vals, uint32_t *tcount,
                        const uint32_t *msrc, const uint32_t *mcom) {
-    // tile position q lives at q + q/32 (one padding word per 32: the
-    // per-thread runs of 16 positions then fall on distinct banks)
-    __shared__ uint32_t rowat[kExpandTile + kExpandTile / 32];
-    __shared__ uint32_t part[kExpandThreads];
-    __shared__ uint32_t r0s, tcnt;
+    __shared__ TileRows rows;
+    __shared__ uint32_t tcnt;
     __shared__ PV wstage[COMBINE ? kExpandThreads : 1];
     const uint32_t t = threadIdx.x;
     static_assert(!(COMBINE && TR), "the member-ordered expansion is not combined");
     if (COMBINE && t == 0) tcnt = 0;
     // the key and graph position of tile position q (edge e)
     auto entry = [&](uint32_t q, uint64_t e, uint64_t &key, uint64_t &p) {
-        const uint32_t r = rowat[q + (q >> 5)];
+        const uint32_t r = rows.row(q);
         if constexpr (TR) {
             p = msrc[r] + (e - off[r]);
             key = ((uint64_t)Cd[__ldcs(col + p)] << bc) | mcom[r];
@@ -83,76 +73,7 @@ __global__ void __launch_bounds__(kExpandThreads)
     };
     for (uint64_t E0 = (uint64_t)blockIdx.x * kExpandTile; E0 < m; E0 += (uint64_t)gridDim.x * kExpandTile) {
         const uint64_t E1 = E0 + kExpandTile < m ? E0 + kExpandTile : m;
-        if (t == 0) {
-            uint32_t lo = 0, hi = n - 1;  // last row with off[row] <= E0: the row of edge E0
-            while (lo < hi) {
-                const uint32_t mid = lo + ((hi - lo + 1) >> 1);
-                if (off[mid] <= E0) lo = mid;
-                else hi = mid - 1;
-            }
-            r0s = lo;
-        }
-        for (uint32_t q = t; q < kExpandTile + kExpandTile / 32; q += kExpandThreads) rowat[q] = 0;
-        __syncthreads();
-        const uint32_t r0 = r0s;
-        if (t == 0) rowat[0] = r0;
-        // rows r0+1, r0+2, ... that start inside the tile, 256 at a time
-        for (uint32_t base = r0 + 1;; base += kExpandThreads) {
-            const uint32_t j = base + t;
-            bool inside = false;
-            if (j < n) {
-                const uint32_t st = off[j];
-                inside = st < E1;
-                if (inside) {
-                    const uint32_t q = (uint32_t)(st - E0);
-                    atomicMax(&rowat[q + (q >> 5)], j);
-                }
-            }
-            // offsets are monotone: more rows can start inside only if the
-            // batch's last one did
-            if (!__syncthreads_or(t == kExpandThreads - 1 && inside)) break;
-        }
-        __syncthreads();
-        // prefix maximum: 16 positions per thread, then across the threads
-        uint32_t run = 0;
-#pragma unroll
-        for (int k = 0; k < kExpandPer; k++) {
-            const uint32_t q = t * kExpandPer + k;
-            run = max(run, rowat[q + (q >> 5)]);
-            rowat[q + (q >> 5)] = run;
-        }
-        part[t] = run;
-        __syncthreads();
-        if (t < 32) {
-            // exclusive prefix maximum of the 256 thread maxima: 8 per lane
-            constexpr int L = kExpandThreads / 32;
-            uint32_t loc[L], v = 0;
-#pragma unroll
-            for (int k = 0; k < L; k++) {
-                v = max(v, part[t * L + k]);
-                loc[k] = v;
-            }
-            uint32_t inc = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if ((int)t >= o) inc = max(inc, y);
-            }
-            uint32_t ex = __shfl_up_sync(0xffffffffu, inc, 1);
-            if (t == 0) ex = 0;
-#pragma unroll
-            for (int k = 0; k < L; k++) part[t * L + k] = k ? max(ex, loc[k - 1]) : ex;
-        }
-        __syncthreads();
-        {
-            const uint32_t pre = part[t];
-#pragma unroll
-            for (int k = 0; k < kExpandPer; k++) {
-                const uint32_t q = t * kExpandPer + k;
-                rowat[q + (q >> 5)] = max(rowat[q + (q >> 5)], pre);
-            }
-        }
-        __syncthreads();
+        tile_rows(off, n, E0, E1, rows);
         if constexpr (!COMBINE) {
 #pragma unroll 4
             for (int k = 0; k < kExpandPer; k++) {
@@ -216,7 +137,7 @@ __global__ void __launch_bounds__(kExpandThreads)
                 tcnt = 0;
             }
         }
-        __syncthreads();  // rowat (and the tile counter) are reused by the next tile
+        __syncthreads();  // the rows (and the tile counter) are reused by the next tile
     }
 }
 
