@@ -37,15 +37,12 @@ mg_status guarded(mg_ctx *ctx, F &&f) {
     }
 }
 
-__global__ void sigma_from_assignment_kernel(const uint32_t *C, const double *k, uint32_t n, double *sigma) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        atomicAdd(sigma + C[v], k[v]);
-}
-
 // copy a host assignment to the device and check every id is < n
 uint32_t *upload_assignment(mg_ctx *ctx, const uint32_t *C, uint32_t n, DBuf<uint32_t> &buf) {
     MG_CHECK(C != nullptr || n == 0, MG_ERR_INVALID, "assignment is NULL");
-    for (uint32_t v = 0; v < n; v++) MG_CHECK(C[v] < n, MG_ERR_INVALID, "community id out of range");
+    uint32_t largest = 0;  // (a loop without exits vectorises)
+    for (uint32_t v = 0; v < n; v++) largest = C[v] > largest ? C[v] : largest;
+    MG_CHECK(n == 0 || largest < n, MG_ERR_INVALID, "community id out of range");
     uint32_t *d = buf.ensure((size_t)n + 1);
     MG_CUDA(cudaMemcpyAsync(d, C, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, ctx->stream));
     return d;
@@ -438,21 +435,10 @@ mg_status mg_modularity(mg_graph *g, const uint32_t *C, double *q) {
         }
         uint32_t *dC = upload_assignment(ctx, C, n, ctx->C[0]);
         uint32_t *dI = ctx->C[2].ensure((size_t)n + 1);
-        uint32_t *dN = ctx->C[1].ensure((size_t)n + 1);
         double *dk = ctx->k.ensure((size_t)n + 1);
         double *ds = ctx->sigma.ensure((size_t)n + 1);
-        level_init(g->view(), dk, ds, dI, s);
-        MG_CUDA(cudaMemsetAsync(ds, 0, sizeof(double) * n, s));
-        sigma_from_assignment_kernel<<<148 * 8, 256, 0, s>>>(dC, dk, n, ds);
-        MG_LAUNCH_CHECK();
-        MoveLevel lvl;
-        move_prepare_level(g->view(), lvl, ctx->mws, s);
-        SweepParams sp;
-        sp.mass = g->mass;
-        sp.integral = g->integral;
         sweep_reset_acc(ctx->mws, s);
-        sigma_sumsq(ds, n, g->integral, ctx->mws, s);
-        move_sweep(g->view(), lvl, ctx->mws, sp, dC, dN, dk, ds, s);  // sums the internal weight of C
+        modularity_terms(g->view(), dC, g->integral, dk, ds, dI, ctx->mws, s);
         MG_CUDA(cudaMemcpyAsync(ctx->h_acc, ctx->mws.acc.get(), sizeof(SweepAcc), cudaMemcpyDeviceToHost, s));
         MG_CUDA(cudaStreamSynchronize(s));
         *q = modularity_from_acc(*ctx->h_acc, g->mass, g->integral);

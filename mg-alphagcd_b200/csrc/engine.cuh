@@ -184,7 +184,8 @@ struct MoveWorkspace {
     DBuf<SweepAcc> tune_acc;       // sums of the autotuner's timing runs (discarded)
     TuneTable tune;
     // the policy is not the default one (mg_sweep_options): every sweep takes
-    // the kernels it names, also on levels that the resident kernel would run
+    // the kernels it names, also on levels that the resident kernels would run
+    // (nor do these run when the caller fixes the shapes, MG_TUNE_OFF / CACHED)
     bool forced_policy = false;
     DBuf<unsigned char> resident;  // resident level kernel: state, sums, counters, barrier
     void *h_resident = nullptr;    // pinned image of them
@@ -301,6 +302,11 @@ void sigma_update(const uint32_t *P, const uint32_t *N, const double *k, double 
                   MoveWorkspace &ws, cudaStream_t s);
 // k_i = row sums; sigma = k; C = identity
 void level_init(const GraphView &g, double *k, double *sigma, uint32_t *C, cudaStream_t s);
+// The sums of the modularity of C into ws.acc (zeroed by the caller): one pass
+// over the edges, without the candidate tables of a sweep.  k, sigma and
+// scratch are work buffers of n entries.
+void modularity_terms(const GraphView &g, const uint32_t *C, int integral, double *k, double *sigma, uint32_t *scratch,
+                      MoveWorkspace &ws, cudaStream_t s);
 // Q = sum_in/mass - s2/mass^2 from host-side copy of the accumulators
 double modularity_from_acc(const SweepAcc &a, double mass, int integral);
 

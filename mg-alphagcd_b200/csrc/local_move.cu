@@ -29,6 +29,7 @@
 // (src/louvain/louvain.cu:105-238), so a separate modularity pass over the
 // edges is not needed.
 #include "lm_kernels.cuh"
+#include "tile_rows.cuh"
 
 namespace mg {
 
@@ -99,27 +100,66 @@ __global__ void sigma_sumsq_kernel(const double *sigma, uint32_t n, int integral
     }
 }
 
+// unit weights: k is the degree, a thread per vertex
+__global__ void level_init_unit_kernel(const uint32_t *off, uint32_t n, double *k, double *sigma, uint32_t *C) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const double s = u2d(off[v + 1] - off[v]);
+        k[v] = s;
+        sigma[v] = s;
+        C[v] = v;
+    }
+}
+
 template <int WK>
 __global__ void level_init_kernel(const uint32_t *off, const void *w, uint32_t n, double *k, double *sigma,
                                   uint32_t *C) {
     // one warp per vertex
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += (gridDim.x * blockDim.x) >> 5) {
-        uint32_t lo = off[v], hi = off[v + 1];
-        double s;
-        if constexpr (WK == WK_UNIT) {
-            s = (double)(hi - lo);
-        } else {
-            s = 0;
-            for (uint32_t e = lo + lane; e < hi; e += 32) s += wload<WK>(w, e);
-            s = warp_sum(s);
-        }
+        const uint32_t lo = off[v], hi = off[v + 1];
+        double s = 0;
+        for (uint32_t e = lo + lane; e < hi; e += 32) s += wload<WK>(w, e);
+        s = warp_sum(s);
         if (lane == 0) {
             k[v] = s;
             sigma[v] = s;
             C[v] = v;
         }
     }
+}
+
+// sigma of an assignment (zeroed by the caller): from k, or (unit weights) from
+// the degrees
+__global__ void sigma_of_kernel(const uint32_t *C, const double *k, const uint32_t *off, uint32_t n, double *sigma) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        atomicAdd(sigma + C[v], k ? k[v] : u2d(off[v + 1] - off[v]));
+}
+
+// Weight of the edges inside a community of C (self-loops included), by tiles
+// of consecutive edges: an edge costs its column and two community gathers,
+// one of them shared by the row.
+template <int WK>
+__global__ void __launch_bounds__(kExpandThreads) inner_weight_kernel(const uint32_t *off, const uint32_t *col,
+                                                                      const void *w, uint32_t n, uint64_t m,
+                                                                      const uint32_t *C, int integral, SweepAcc *acc) {
+    __shared__ TileRows rows;
+    double sin = 0;
+    for (uint64_t E0 = (uint64_t)blockIdx.x * kExpandTile; E0 < m; E0 += (uint64_t)gridDim.x * kExpandTile) {
+        const uint64_t E1 = E0 + kExpandTile < m ? E0 + kExpandTile : m;
+        tile_rows(off, n, E0, E1, rows);
+#pragma unroll 8
+        for (int k = 0; k < kExpandPer; k++) {
+            const uint32_t q = k * kExpandThreads + threadIdx.x;
+            const uint64_t e = E0 + q;
+            if (e < E1) {
+                const bool in = C[__ldcs(col + e)] == C[rows.row(q)];
+                if constexpr (WK == WK_UNIT) sin += in ? 1.0 : 0.0;
+                else sin += in ? wload<WK>(w, (uint32_t)e) : 0.0;
+            }
+        }
+        __syncthreads();  // the rows are filled again
+    }
+    flush_acc(acc, integral, sin, 0);
 }
 
 // Largest cluster size (8 or 16) the device schedules for the heavy tiers.
@@ -304,11 +344,35 @@ void sigma_update(const uint32_t *P, const uint32_t *N, const double *k, double 
 void level_init(const GraphView &g, double *k, double *sigma, uint32_t *C, cudaStream_t s) {
     if (g.n == 0) return;
     unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(g.n, 8), 148ull * 16);
-    if (g.wk == WK_UNIT) level_init_kernel<WK_UNIT><<<grid, 256, 0, s>>>(g.off, g.w, g.n, k, sigma, C);
+    if (g.wk == WK_UNIT)
+        level_init_unit_kernel<<<(unsigned)std::min<uint64_t>(ceil_div(g.n, 256), 148ull * 16), 256, 0, s>>>(
+            g.off, g.n, k, sigma, C);
     else if (g.wk == WK_F32) level_init_kernel<WK_F32><<<grid, 256, 0, s>>>(g.off, g.w, g.n, k, sigma, C);
     else if (g.wk == WK_U32) level_init_kernel<WK_U32><<<grid, 256, 0, s>>>(g.off, g.w, g.n, k, sigma, C);
     else level_init_kernel<WK_F64><<<grid, 256, 0, s>>>(g.off, g.w, g.n, k, sigma, C);
     MG_LAUNCH_CHECK();
+}
+
+void modularity_terms(const GraphView &g, const uint32_t *C, int integral, double *k, double *sigma, uint32_t *scratch,
+                      MoveWorkspace &ws, cudaStream_t s) {
+    if (g.n == 0) return;
+    if (g.wk != WK_UNIT) level_init(g, k, sigma, scratch, s);
+    MG_CUDA(cudaMemsetAsync(sigma, 0, sizeof(double) * g.n, s));
+    sigma_of_kernel<<<(unsigned)std::min<uint64_t>(ceil_div(g.n, 256), 148ull * 8), 256, 0, s>>>(
+        C, g.wk != WK_UNIT ? k : nullptr, g.off, g.n, sigma);
+    MG_LAUNCH_CHECK();
+    sigma_sumsq(sigma, g.n, integral, ws, s);
+    if (g.nnz == 0) return;
+    SweepAcc *acc = ws.acc.ensure(1);
+    const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(g.nnz, kExpandTile), 148ull * 8);
+    auto run = [&](auto kern) {
+        kern<<<grid, kExpandThreads, 0, s>>>(g.off, g.col, g.w, g.n, g.nnz, C, integral, acc);
+        MG_LAUNCH_CHECK();
+    };
+    if (g.wk == WK_UNIT) run(inner_weight_kernel<WK_UNIT>);
+    else if (g.wk == WK_F32) run(inner_weight_kernel<WK_F32>);
+    else if (g.wk == WK_U32) run(inner_weight_kernel<WK_U32>);
+    else run(inner_weight_kernel<WK_F64>);
 }
 
 double modularity_from_acc(const SweepAcc &a, double mass, int integral) {
