@@ -601,7 +601,7 @@ class Batch:
                 for f, _ in _BatchGraph._fields_:
                     per[f].append(getattr(bg, f))
                 if assignments:
-                    a = np.zeros(max(bg.n, 1), np.uint32)
+                    a = np.empty(max(bg.n, 1), np.uint32)
                     lib().mg_batch_result_assignment(r, g, _p(a))
                     assign.append(a[: bg.n])
             out["graphs"] = {f: np.array(v) for f, v in per.items()}
@@ -702,7 +702,7 @@ class Graph:
             s = _Summary()
             lib().mg_result_summary(r, ct.byref(s))
             n = self.info()["n"]
-            a = np.zeros(max(n, 1), np.uint32)
+            a = np.empty(max(n, 1), np.uint32)
             lib().mg_result_assignment(r, _p(a))
             cnt = ct.c_int()
             lib().mg_result_level_sizes(r, None, 0, ct.byref(cnt))

@@ -630,7 +630,7 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
     res.graphs = G;
     res.voff = b->voff;
     res.per.assign(G, mg_batch_graph_summary{});
-    res.assignment.assign(n0, 0);
+    res.assignment.ensure(n0, ctx->spare);
     mg_summary &S = res.sum;
     // graphs without edges keep the identity (as mg_louvain_run does)
     std::vector<uint8_t> alive(G, 0);

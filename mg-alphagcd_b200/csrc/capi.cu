@@ -144,7 +144,7 @@ mg_status mg_graph_from_csr(mg_ctx *ctx, uint32_t n, const uint64_t *offsets, co
     *out = nullptr;
     mg_graph *g = new (std::nothrow) mg_graph();
     if (!g) return fail(ctx, MG_ERR_OOM, "host allocation failed");
-    g->ctx = ctx;
+    g->attach(ctx);
     mg_status st = guarded(ctx, [&] { graph_from_host_csr(g, n, offsets, cols, weights, weight_type); });
     if (st != MG_OK) {
         delete g;
@@ -160,7 +160,7 @@ mg_status mg_graph_from_device_csr(mg_ctx *ctx, uint32_t n, uint64_t nnz, const 
     *out = nullptr;
     mg_graph *g = new (std::nothrow) mg_graph();
     if (!g) return fail(ctx, MG_ERR_OOM, "host allocation failed");
-    g->ctx = ctx;
+    g->attach(ctx);
     mg_status st = guarded(ctx, [&] { graph_from_device_csr(g, n, nnz, d_offsets32, d_cols, d_weights, weight_type); });
     if (st != MG_OK) {
         delete g;
@@ -238,7 +238,7 @@ mg_status mg_graph_generate_rmat(mg_ctx *ctx, int scale, int edge_factor, double
     *out = nullptr;
     mg_graph *g = new (std::nothrow) mg_graph();
     if (!g) return fail(ctx, MG_ERR_OOM, "host allocation failed");
-    g->ctx = ctx;
+    g->attach(ctx);
     mg_status st = guarded(ctx, [&] { graph_generate_rmat(g, scale, edge_factor, a, b, c, seed); });
     if (st != MG_OK) {
         delete g;
@@ -254,7 +254,7 @@ mg_status mg_graph_generate_sbm(mg_ctx *ctx, uint32_t n, uint32_t blocks, double
     *out = nullptr;
     mg_graph *g = new (std::nothrow) mg_graph();
     if (!g) return fail(ctx, MG_ERR_OOM, "host allocation failed");
-    g->ctx = ctx;
+    g->attach(ctx);
     mg_status st = guarded(ctx, [&] { graph_generate_sbm(g, n, blocks, mean_degree, intra_frac, seed); });
     if (st != MG_OK) {
         delete g;
@@ -270,7 +270,7 @@ mg_status mg_graph_generate_chunglu(mg_ctx *ctx, uint32_t n, double exponent, do
     *out = nullptr;
     mg_graph *g = new (std::nothrow) mg_graph();
     if (!g) return fail(ctx, MG_ERR_OOM, "host allocation failed");
-    g->ctx = ctx;
+    g->attach(ctx);
     mg_status st = guarded(ctx, [&] { graph_generate_chunglu(g, n, exponent, mean_degree, max_degree, lognormal, seed); });
     if (st != MG_OK) {
         delete g;
@@ -367,7 +367,7 @@ mg_status mg_bins_offsets(mg_ctx *ctx, int scheme, uint32_t n, const uint64_t *o
             MG_CHECK(i == 0 || offsets[i] >= offsets[i - 1], MG_ERR_INVALID, "offsets must be non-decreasing");
             o32[i] = (uint32_t)offsets[i];
         }
-        DBuf<uint32_t> d_off;
+        DBuf<uint32_t> d_off(&ctx->pool);
         uint32_t *d = d_off.ensure((size_t)n + 1);
         MG_CUDA(cudaMemcpyAsync(d, o32.data(), sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, ctx->stream));
         uint32_t *d_perm = ctx->tmp32.ensure((size_t)n + 1);
@@ -451,7 +451,7 @@ mg_status mg_coarsen(mg_graph *g, const uint32_t *C, uint32_t *C_dense, mg_graph
     mg_ctx *ctx = g->ctx;
     mg_graph *ng = new (std::nothrow) mg_graph();
     if (!ng) return fail(ctx, MG_ERR_OOM, "host allocation failed");
-    ng->ctx = ctx;
+    ng->attach(ctx);
     mg_status st = guarded(ctx, [&] {
         ctx_prepare(ctx);
         cudaStream_t s = ctx->stream;
@@ -459,7 +459,7 @@ mg_status mg_coarsen(mg_graph *g, const uint32_t *C, uint32_t *C_dense, mg_graph
         uint32_t *dC = upload_assignment(ctx, C, n, ctx->C[0]);
         uint32_t *dCd = ctx->Cd.ensure((size_t)n + 1);
         uint32_t nn = relabel_dense(dC, n, dCd, ctx->cws, s);
-        LevelGraph lv;
+        LevelGraph lv(&ctx->pool);
         coarsen_level(g->view(), dCd, nn, g->integral, lv, ctx->cws, s, nullptr,
                       ctx->mws.coarsen_combine == MG_COMBINE_ON);
         if (C_dense && n) {

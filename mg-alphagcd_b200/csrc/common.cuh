@@ -6,8 +6,11 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "../../include/mgagcd.h"
 
@@ -68,17 +71,74 @@ inline uint32_t pow2_at_least(uint64_t x, uint32_t lo = 16) {
 // as out of memory, once.  Process-wide.
 bool alloc_fault_due();
 
-// Grow-only device allocation owned by the engine (cudaMalloc on growth only).
+// Device buffers of graphs that ended, kept by their context for the next ones:
+// a graph that is uploaded, used once and dropped otherwise pays a cudaMalloc
+// and a cudaFree (which waits for the device) per array.  At most kBytes and
+// kCount buffers are kept; they go back when the context ends or an allocation
+// finds no memory.  All work on a context's buffers is ordered by its stream,
+// so a buffer may be handed out while kernels of its last user still run.
+class BufPool {
+public:
+    static constexpr size_t kBytes = 256u << 20;
+    static constexpr size_t kCount = 32;
+    BufPool() = default;
+    BufPool(const BufPool &) = delete;
+    BufPool &operator=(const BufPool &) = delete;
+    ~BufPool() { trim(); }
+    // the smallest kept buffer of at least `bytes` and not far above; null: none
+    void *take(size_t bytes, size_t &got) {
+        std::lock_guard<std::mutex> lk(mu_);
+        size_t best = kept_.size();
+        for (size_t i = 0; i < kept_.size(); i++)
+            if (kept_[i].second >= bytes && kept_[i].second <= 2 * bytes + 65536 &&
+                (best == kept_.size() || kept_[i].second < kept_[best].second))
+                best = i;
+        if (best == kept_.size()) return nullptr;
+        void *p = kept_[best].first;
+        got = kept_[best].second;
+        total_ -= got;
+        kept_.erase(kept_.begin() + (long)best);
+        return p;
+    }
+    void give(void *p, size_t bytes) {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (total_ + bytes <= kBytes && kept_.size() < kCount) {
+                kept_.emplace_back(p, bytes);
+                total_ += bytes;
+                return;
+            }
+        }
+        cudaFree(p);
+    }
+    void trim() {
+        std::lock_guard<std::mutex> lk(mu_);
+        for (auto &b : kept_) cudaFree(b.first);
+        kept_.clear();
+        total_ = 0;
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<std::pair<void *, size_t>> kept_;
+    size_t total_ = 0;
+};
+
+// Grow-only device allocation owned by the engine (cudaMalloc on growth only),
+// from and back to a pool where it has one.
 template <class T>
 struct DBuf {
     T *p = nullptr;
     size_t cap = 0;
+    BufPool *pool = nullptr;
     DBuf() = default;
+    explicit DBuf(BufPool *from) : pool(from) {}
     DBuf(const DBuf &) = delete;
     DBuf &operator=(const DBuf &) = delete;
     ~DBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p && pool) pool->give(p, cap * sizeof(T));
+        else if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
     }
@@ -87,7 +147,17 @@ struct DBuf {
             release();
             size_t want = n < 16 ? 16 : n;
             if (alloc_fault_due()) throw Error(MG_ERR_OOM, "device allocation failed (injected by mg_test_fail_allocation)");
-            MG_CUDA(cudaMalloc(&p, want * sizeof(T)));
+            size_t got = 0;
+            if (pool && (p = (T *)pool->take(want * sizeof(T), got))) {
+                cap = got / sizeof(T);
+                return p;
+            }
+            if (pool && cudaMalloc(&p, want * sizeof(T)) != cudaSuccess) {
+                cudaGetLastError();  // once more with what the pool holds given back
+                p = nullptr;
+                pool->trim();
+            }
+            if (!p) MG_CUDA(cudaMalloc(&p, want * sizeof(T)));
             cap = want;
         }
         return p;

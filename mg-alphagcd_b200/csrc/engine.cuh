@@ -314,9 +314,9 @@ double modularity_from_acc(const SweepAcc &a, double mass, int integral);
 // line lies where the two paths meet: one CTA per SM keeps fewer warps in
 // flight than the class kernels, which counts once a sweep takes longer than
 // their launches.  SBM runs, local move only, resident / class kernels: 1.0 M
-// entries 2.9 / 6.0 ms, 4.0 M 6.9 / 9.4, 10 M 15.7 / 16.7, 24 M 38.7 / 31.5;
-// Chung-Lu, 15 M entries: 16.8 / 19.1 ms.
-constexpr uint64_t kResidentMaxEntries = 12u << 20;
+// entries 2.5 / 5.5 ms, 4.0 M 5.2 / 8.1, 10 M 11.7 / 14.4, 24 M 29.0 / 25.7;
+// Chung-Lu, 15 M entries: 15.2 / 17.5 ms.
+constexpr uint64_t kResidentMaxEntries = 20u << 20;
 struct ResidentResult {
     int base = 0;                            // buffer holding the accepted assignment
     std::vector<double> Q;                   // per sweep: Q of its input assignment
@@ -351,6 +351,8 @@ struct LevelGraph {
     DBuf<uint32_t> off, col;
     DBuf<double> w;
     DBuf<uint32_t> wi;
+    LevelGraph() = default;
+    explicit LevelGraph(BufPool *pool) : off(pool), col(pool), w(pool), wi(pool) {}
     int wk = WK_F64;
     bool symmetric = false;  // coarsened from a symmetric integral graph
     GraphView view() const {

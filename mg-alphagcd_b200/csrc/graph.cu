@@ -269,10 +269,11 @@ __global__ void weight_stats_kernel(const T *w, uint64_t m, double *partial, int
 
 // mass and integrality of a device weight array (deterministic block order)
 template <class T>
-static void device_weight_stats(const T *w, uint64_t m, double &mass, int &integral, int &unit, cudaStream_t s) {
+static void device_weight_stats(const T *w, uint64_t m, double &mass, int &integral, int &unit, mg_ctx *ctx) {
+    cudaStream_t s = ctx->stream;
     const unsigned blocks = 148 * 4;
-    DBuf<double> part;
-    DBuf<int> flags;
+    DBuf<double> part(&ctx->pool);
+    DBuf<int> flags(&ctx->pool);
     double *p = part.ensure(blocks);
     int *f = flags.ensure(2);
     MG_CUDA(cudaMemsetAsync(f, 0, 2 * sizeof(int), s));
@@ -297,7 +298,7 @@ static void detect_row_properties(mg_graph *g, cudaStream_t s) {
     g->sorted_rows = 1;
     g->symmetric = g->integral;
     if (g->n == 0) return;
-    DBuf<unsigned long long> flags;
+    DBuf<unsigned long long> flags(&g->ctx->pool);
     unsigned long long *d = flags.ensure(5);
     MG_CUDA(cudaMemsetAsync(d, 0, 5 * sizeof(unsigned long long), s));
     int *uns = (int *)(d + 4);
@@ -344,8 +345,8 @@ void graph_from_host_csr(mg_graph *g, uint32_t n, const uint64_t *offsets, const
     g->nnz = nnz;
     // offsets and columns are checked on the device after the copy
     {
-        DBuf<uint64_t> off64;
-        DBuf<int> bad;
+        DBuf<uint64_t> off64(&g->ctx->pool);
+        DBuf<int> bad(&g->ctx->pool);
         uint64_t *d64 = off64.ensure((size_t)n + 1);
         int *dbad = bad.ensure(1);
         MG_CUDA(cudaMemsetAsync(dbad, 0, sizeof(int), s));
@@ -391,13 +392,13 @@ void graph_from_device_csr(mg_graph *g, uint32_t n, uint64_t nnz, const uint32_t
     if (weight_type != MG_WEIGHT_UNIT && nnz > 0) {
         int integral = 0, unit = 0;
         if (weight_type == MG_WEIGHT_F32) {
-            device_weight_stats<float>((const float *)d_w, nnz, g->mass, integral, unit, s);
+            device_weight_stats<float>((const float *)d_w, nnz, g->mass, integral, unit, g->ctx);
             if (!unit) {
                 g->wk = WK_F32;
                 MG_CUDA(cudaMemcpyAsync(g->w32.ensure(nnz + 1), d_w, sizeof(float) * nnz, cudaMemcpyDeviceToDevice, s));
             }
         } else {
-            device_weight_stats<double>((const double *)d_w, nnz, g->mass, integral, unit, s);
+            device_weight_stats<double>((const double *)d_w, nnz, g->mass, integral, unit, g->ctx);
             if (!unit) {
                 g->wk = WK_F64;
                 MG_CUDA(cudaMemcpyAsync(g->w64.ensure(nnz + 1), d_w, sizeof(double) * nnz, cudaMemcpyDeviceToDevice, s));
@@ -431,7 +432,7 @@ void graph_from_level(mg_graph *g, LevelGraph &lv, int integral, double mass) {
 static void finish_generated(mg_graph *g, uint32_t n, uint64_t m, DBuf<uint32_t> &u, DBuf<uint32_t> &v) {
     mg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
-    LevelGraph lv;
+    LevelGraph lv(&ctx->pool);
     csr_from_device_pairs(n, m, u.get(), v.get(), lv, ctx->cws, s);
     u.release();
     v.release();
@@ -460,7 +461,7 @@ void graph_generate_rmat(mg_graph *g, int scale, int edge_factor, double a, doub
     const uint64_t t2 = (uint64_t)((a + b) * 4294967296.0);
     const uint64_t t3 = (uint64_t)((a + b + c) * 4294967296.0);
     const uint64_t key = rng_key(seed, 0x524d4154ull);
-    DBuf<uint32_t> u, v;
+    DBuf<uint32_t> u(&g->ctx->pool), v(&g->ctx->pool);
     u.ensure(m);
     v.ensure(m);
     cudaStream_t s = g->ctx->stream;
@@ -478,7 +479,7 @@ void graph_generate_sbm(mg_graph *g, uint32_t n, uint32_t blocks, double mean_de
     const uint64_t mout = blocks > 1 ? (uint64_t)std::llround((double)n * dout / 2.0) : 0;
     const uint64_t m = min_ + mout;
     MG_CHECK(2 * m < 0xFFFFFFFFull, MG_ERR_UNSUPPORTED, "sbm: more than 2^32-1 directed entries");
-    DBuf<uint32_t> u, v;
+    DBuf<uint32_t> u(&g->ctx->pool), v(&g->ctx->pool);
     u.ensure(m + 1);
     v.ensure(m + 1);
     cudaStream_t s = g->ctx->stream;
@@ -539,9 +540,9 @@ void graph_generate_chunglu(mg_graph *g, uint32_t n, double exponent, double mea
     MG_CHECK(2 * m < 0xFFFFFFFFull, MG_ERR_UNSUPPORTED, "chung-lu: more than 2^32-1 directed entries");
     mg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
-    DBuf<uint64_t> dcdf;
-    DBuf<uint32_t> u, v;
-    DBuf<double> w;
+    DBuf<uint64_t> dcdf(&ctx->pool);
+    DBuf<uint32_t> u(&ctx->pool), v(&ctx->pool);
+    DBuf<double> w(&ctx->pool);
     MG_CUDA(cudaMemcpyAsync(dcdf.ensure(n), cdf.data(), sizeof(uint64_t) * n, cudaMemcpyHostToDevice, s));
     u.ensure(m + 1);
     v.ensure(m + 1);
@@ -551,7 +552,7 @@ void graph_generate_chunglu(mg_graph *g, uint32_t n, double exponent, double mea
                                                       rng_key(seed, 0x4c4f474eull), u.get(), v.get(), dw);
         MG_LAUNCH_CHECK();
     }
-    LevelGraph lv;
+    LevelGraph lv(&ctx->pool);
     csr_from_device_pairs(n, m, u.get(), v.get(), lv, ctx->cws, s, dw);
     g->n = n;
     g->nnz = lv.nnz;
@@ -573,7 +574,7 @@ void graph_generate_chunglu(mg_graph *g, uint32_t n, double exponent, double mea
         }
         g->wk = WK_F32;
         int integral = 0, unit = 0;
-        device_weight_stats<float>(g->w32.get(), lv.nnz, g->mass, integral, unit, s);
+        device_weight_stats<float>(g->w32.get(), lv.nnz, g->mass, integral, unit, g->ctx);
         g->integral = integral;
     }
     g->symmetric = g->integral;  // both directions of every pair, with its weight

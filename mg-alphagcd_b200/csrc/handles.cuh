@@ -2,17 +2,118 @@
 // mg_result) and the engine entry points the ABI calls.
 #pragma once
 
+#include <cstdlib>
 #include <functional>
+#include <memory>
+#include <mutex>
+#include <new>
 #include <string>
+#include <algorithm>
 #include <vector>
 
 #include "engine.cuh"
+
+namespace mg {
+// Host memory of a result's assignment.  A context keeps one page-locked buffer
+// (at most kPinnedIds ids) that the result it is lent to gives back when it
+// ends, also after the context: a copy of 64 MB into it runs at the link's
+// speed, where fresh pageable memory costs its page faults and a staged copy
+// (R-MAT-24: 25 of 45 ms of host time beside a run).  While it is lent out,
+// further results take plain memory.
+constexpr size_t kPinnedIds = 64u << 20;
+struct PinnedSpare {
+    std::mutex mu;
+    uint32_t *p = nullptr;
+    size_t cap = 0;
+    ~PinnedSpare() {
+        if (p) cudaFreeHost(p);
+    }
+};
+class HostIds {
+public:
+    HostIds() = default;
+    HostIds(const HostIds &) = delete;
+    HostIds &operator=(const HostIds &) = delete;
+    HostIds(HostIds &&o) noexcept { swap(o); }
+    HostIds &operator=(HostIds &&o) noexcept {
+        swap(o);
+        return *this;
+    }
+    ~HostIds() { release(); }
+    // n uninitialised ids; does nothing when they are there already
+    void ensure(size_t n, const std::shared_ptr<PinnedSpare> &spare) {
+        if (p_ && n_ == n) return;
+        release();
+        if (n >= kPinnedFrom && n <= kPinnedIds) {
+            std::lock_guard<std::mutex> lk(spare->mu);
+            if (!lent_ok(*spare, n)) return plain(n);
+            p_ = spare->p;
+            cap_ = spare->cap;
+            spare->p = nullptr;
+            spare->cap = kLent;
+            spare_ = spare;
+            n_ = n;
+            return;
+        }
+        plain(n);
+    }
+    uint32_t *data() { return p_; }
+    const uint32_t *data() const { return p_; }
+    uint32_t &operator[](size_t i) { return p_[i]; }
+
+private:
+    static constexpr size_t kPinnedFrom = 1u << 18;  // smaller copies cost less than the lending
+    uint32_t *p_ = nullptr;
+    size_t n_ = 0, cap_ = 0;
+    std::shared_ptr<PinnedSpare> spare_;  // set: p_ is its buffer
+    void swap(HostIds &o) {
+        std::swap(p_, o.p_);
+        std::swap(n_, o.n_);
+        std::swap(cap_, o.cap_);
+        spare_.swap(o.spare_);
+    }
+    // the spare buffer is there and large enough (made or grown here unless lent)
+    static bool lent_ok(PinnedSpare &s, size_t n) {
+        if (s.p && s.cap >= n) return true;
+        if (!s.p && s.cap == kLent) return false;
+        if (s.p) cudaFreeHost(s.p);
+        s.p = nullptr;
+        s.cap = 0;
+        if (cudaMallocHost(&s.p, n * sizeof(uint32_t)) != cudaSuccess) {
+            cudaGetLastError();  // no page-locked memory: plain memory serves
+            s.p = nullptr;
+            return false;
+        }
+        s.cap = n;
+        return true;
+    }
+    void plain(size_t n) {
+        p_ = (uint32_t *)malloc(std::max<size_t>(n, 1) * sizeof(uint32_t));
+        if (!p_) throw std::bad_alloc();
+        n_ = n;
+    }
+    void release() {
+        if (spare_) {
+            std::lock_guard<std::mutex> lk(spare_->mu);
+            spare_->p = p_;
+            spare_->cap = cap_;
+        } else {
+            free(p_);
+        }
+        spare_.reset();
+        p_ = nullptr;
+        n_ = cap_ = 0;
+    }
+    static constexpr size_t kLent = ~(size_t)0;  // PinnedSpare::cap while a result holds the buffer
+};
+}  // namespace mg
 
 struct mg_ctx {
     int device = 0;
     int verbose = 0;
     size_t budget = 0;
     std::string last_error;
+    mg::BufPool pool;  // (before the buffers that return to it)
     cudaStream_t stream = nullptr;
     mg::MoveWorkspace mws;
     mg::CoarsenWorkspace cws;
@@ -21,6 +122,7 @@ struct mg_ctx {
     mg::DBuf<double> k, sigma;
     mg::LevelGraph lv[2];
     mg::SweepAcc *h_acc = nullptr;  // pinned
+    std::shared_ptr<mg::PinnedSpare> spare = std::make_shared<mg::PinnedSpare>();
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     ~mg_ctx();
 };
@@ -36,6 +138,12 @@ struct mg_graph {
     double mass = 0;
     int integral = 1;
     int sorted_rows = 0;  // every row strictly increasing (no repeated neighbour)
+    void attach(mg_ctx *c) {  // the context and its buffer pool
+        ctx = c;
+        off.pool = col.pool = &c->pool;
+        w32.pool = &c->pool;
+        w64.pool = &c->pool;
+    }
     int symmetric = 0;    // integral and symmetric as a multiset of entries (GraphView::symmetric)
     mg::GraphView view() const {
         mg::GraphView v;
@@ -54,7 +162,7 @@ struct mg_graph {
 struct mg_result {
     uint32_t n0 = 0;
     mg_summary sum{};
-    std::vector<uint32_t> assignment;
+    mg::HostIds assignment;
     std::vector<uint32_t> level_sizes;
     std::vector<double> trace;  // rows of 4
     std::vector<std::vector<uint32_t>> level_maps;  // dendrogram (keep_levels)
@@ -128,7 +236,7 @@ struct mg_batch_result {
     mg_summary sum{};
     std::vector<mg_batch_graph_summary> per;
     std::vector<uint32_t> voff;        // first vertex of each graph
-    std::vector<uint32_t> assignment;  // graph-local community of every packed vertex
+    mg::HostIds assignment;            // graph-local community of every packed vertex
 };
 
 namespace mg {

@@ -95,9 +95,9 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
     const bool verbose = o.verbose || ctx->verbose;
     res = mg_result();
     res.n0 = n0;
-    res.assignment.assign(n0, 0);
     mg_summary &S = res.sum;
     if (n0 == 0 || g->nnz == 0 || mass <= 0) {
+        res.assignment.ensure(n0, ctx->spare);
         for (uint32_t v = 0; v < n0; v++) res.assignment[v] = v;
         S.communities = n0;
         return;
@@ -185,6 +185,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
             move_sweep(cur, mlv, ctx->mws, sp, C[base], C[pend], k, sigma, s);
             MG_CUDA(cudaEventRecord(ctx->ev[5], s));
             MG_CUDA(cudaMemcpyAsync(&hacc, ctx->mws.acc.get(), sizeof(SweepAcc), cudaMemcpyDeviceToHost, s));
+            res.assignment.ensure(n0, ctx->spare);  // (while the sweep runs)
             double lm = tp.stop_sync();
             phase_lm += lm;
             account_sweep(ctx, cur, hacc, S);
@@ -263,6 +264,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         phase++;
     }
     MG_CUDA(cudaEventRecord(ctx->ev[3], s));
+    res.assignment.ensure(n0, ctx->spare);
     MG_CUDA(cudaMemcpyAsync(res.assignment.data(), assign, sizeof(uint32_t) * n0, cudaMemcpyDeviceToHost, s));
     MG_CUDA(cudaStreamSynchronize(s));
     float ms = 0;
