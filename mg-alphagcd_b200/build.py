@@ -22,7 +22,7 @@ CXXFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler
             "-ccbin", "/usr/bin/g++", "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include")]
 SOURCES = ["primitives.cu", "bins.cu", "local_move.cu", "local_move_batch.cu", "coarsen.cu", "graph.cu",
            "louvain.cu", "batch.cu", "serve.cu", "capi.cu",
-           "mtx.cpp", "noalloc.cu", "resident.cu", "resident_unit.cu", "resident_u32.cu", "resident_f32i.cu",
+           "mtx.cpp", "noalloc.cu", "resident.cu", "small_level.cu", "resident_unit.cu", "resident_u32.cu", "resident_f32i.cu",
            "resident_f64i.cu", "resident_f32.cu", "resident_f64.cu"]
 LIB = os.path.join(HERE, "libmgagcd.so")
 CLI = os.path.join(HERE, "MG_GCD")

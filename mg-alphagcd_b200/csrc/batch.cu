@@ -498,14 +498,16 @@ __global__ void class_starts_kernel(const uint32_t *perm, Idx19 off, const uint3
 // CTAs per graph for a phase of the resident kernel, 0 when the class kernels
 // serve it better.  Both are estimated per sweep: a CTA sweeps kSmRate entries
 // per microsecond and a sweep takes kSweepMin at least; clusters take the graphs
-// in turn, largest first, so a phase ends after the mean load of a cluster plus
-// at most one graph.  The class kernels sweep kClassRate entries per microsecond
-// over all graphs and pay kClassSweep per sweep for launches and the per-graph
-// sums.  (One graph among many that is too large for a cluster, or a vertex
-// of more communities than a CTA's table holds, sends the phase there.)
+// in turn, largest first, so a phase ends near the larger of the mean load of a
+// cluster and the largest graph's (a third of the smaller is added for graphs that
+// take more iterations than others).  The class kernels sweep kClassRate
+// entries per microsecond over all graphs and pay kClassSweep per sweep for
+// launches and the per-graph sums.  (One graph among many that is too large for
+// a cluster, or a vertex of more communities than a CTA's table holds, sends
+// the phase there.)
 int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vector<uint32_t> &alive,
                   const std::vector<uint64_t> &load, uint32_t most_vertices) {
-    constexpr double kSmRate = 365, kSweepMin = 8, kClassRate = 42e3, kClassSweep = 120;
+    constexpr double kSmRate = 440, kSweepMin = 8, kClassRate = 46e3, kClassSweep = 120;
     if (ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
     if (std::min(lvl.bins.max_degree, most_vertices) > lmr::kResidentCapacity) return 0;
     double total = 0;
@@ -520,7 +522,7 @@ int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vect
             most = std::max(most, t);
         }
         const double clusters = kNumSMs / cs;
-        const double est = std::max(most, sum / clusters + most * (1 - 1 / clusters));
+        const double mean = sum / clusters, est = std::max(most, mean) + 0.35 * std::min(most, mean);
         if (est < best) {
             best = est;
             ctas = cs;

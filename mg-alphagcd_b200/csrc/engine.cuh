@@ -160,6 +160,13 @@ struct TuneTable {
 };
 constexpr uint32_t kTuneMinVertices = 4096;  // smaller classes keep the default shape
 
+// From one small level to the next in one launch (small_level.cu).
+constexpr uint32_t kSmallEntries = 8192;  // most vertices and entries of such a level
+struct SmallInfo {
+    uint32_t n, nnz, max_degree;
+    uint32_t size[kSweepClasses], offset[kSweepClasses];
+};
+
 struct MoveWorkspace {
     DBuf<uint32_t> perm;
     DBuf<uint2> rows;              // {off[perm[q]], off[perm[q] + 1]} per class-list entry q
@@ -189,6 +196,7 @@ struct MoveWorkspace {
     bool forced_policy = false;
     DBuf<unsigned char> resident;  // resident level kernel: state, sums, counters, barrier
     void *h_resident = nullptr;    // pinned image of them
+    DBuf<SmallInfo> small;         // counts of a small level
     PrimWorkspace prim;
     // stream 0: heavy tiers; streams 1..light_streams: the light classes and
     // the class-13 tier, so that one class's tail overlaps the others (one by
@@ -370,6 +378,13 @@ struct LevelGraph {
 };
 // The weights of a level as doubles (device, nnz entries).
 void level_weights_f64(const GraphView &g, double *out, cudaStream_t s);
+// A level of at most kSmallEntries vertices and entries: dense relabel of C
+// into Cd (n_new communities) and, with coarsen, the next level with its vertex
+// weights, singletons (ctx->k, sigma, C[0]) and degree classes -- what
+// relabel_dense, coarsen_level, level_init and move_prepare_level give, except
+// that a class lists its vertices in any order (the resident kernel's input).
+void small_level(mg_ctx *ctx, const GraphView &g, const uint32_t *C, uint32_t *Cd, bool coarsen, int integral,
+                 LevelGraph &out, MoveLevel &lvl, uint32_t &n_new, cudaStream_t s);
 // Dense order-preserving relabel; returns n'.
 uint32_t relabel_dense(const uint32_t *C, uint32_t n, uint32_t *C_dense, CoarsenWorkspace &ws, cudaStream_t s);
 // Next level from a graph and a dense assignment with n' communities.

@@ -117,6 +117,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
     double Qh = 0, Qold = -1;
     int phase = 0;
     MoveLevel mlv;
+    bool prepared = false;  // the level's start came with its coarsening (small levels)
     SweepParams sp;
     sp.version = version;
     sp.precision = o.precision;
@@ -133,8 +134,12 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         if (verbose) print_phase_header(phase);
         double phase_lm = 0;
         Timer tp(ctx->ev[0], ctx->ev[1], s);
-        level_init(cur, k, sigma, C[0], s);
-        move_prepare_level(cur, mlv, ctx->mws, s);
+        if (!prepared) {
+            level_init(cur, k, sigma, C[0], s);
+            move_prepare_level(cur, mlv, ctx->mws, s);
+        }
+        prepared = false;
+        bool resident = false;
         int base = 0, loop = 0;
         double curQ = 0;
         unsigned long long last_distinct = 0;
@@ -148,6 +153,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         // (the printed table has a time per iteration: verbose runs take the
         // iteration-by-iteration path)
         if (!verbose && resident_level(cur, mlv, ctx->mws)) {
+            resident = true;
             ResidentResult R;
             MG_CUDA(cudaEventRecord(ctx->ev[4], s));
             resident_run(ctx, cur, mlv, sp, thr, R, s);
@@ -243,19 +249,27 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         // dense relabel of the final assignment of this phase, composed into
         // the assignment of the input vertices
         Timer tc(ctx->ev[0], ctx->ev[1], s);
-        const uint32_t nn = relabel_dense(C[base], n, Cd, ctx->cws, s);
+        // (a small level is followed by another one, which the resident kernel
+        // takes too: relabelled, coarsened and prepared in one launch)
+        const bool last = (Qh - Qold) <= thr;
+        const bool small = resident && n <= kSmallEntries && cur.nnz <= kSmallEntries;
+        uint32_t nn;
+        if (small) small_level(ctx, cur, C[base], Cd, !last, integral, ctx->lv[lvl_out], mlv, nn, s);
+        else nn = relabel_dense(C[base], n, Cd, ctx->cws, s);
         gather_compose(assign, Cd, n0, s);
         if (o.keep_levels) {
             res.level_maps.emplace_back(n);
             MG_CUDA(cudaMemcpyAsync(res.level_maps.back().data(), Cd, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s));
         }
         communities = nn;
-        if ((Qh - Qold) <= thr) {
+        if (last) {
             S.seconds_coarsen += tc.stop_sync();
             break;
         }
-        coarsen_level(cur, Cd, nn, integral, ctx->lv[lvl_out], ctx->cws, s, nullptr,
-                      coarsen_combine(ctx->mws, last_distinct, cur.nnz));
+        prepared = small;
+        if (!small)
+            coarsen_level(cur, Cd, nn, integral, ctx->lv[lvl_out], ctx->cws, s, nullptr,
+                          coarsen_combine(ctx->mws, last_distinct, cur.nnz));
         double ct = tc.stop_sync();
         S.seconds_coarsen += ct;
         if (verbose) printf("Coarsen graph execution time: %f s, %f ms\n", ct, ct * 1e3);

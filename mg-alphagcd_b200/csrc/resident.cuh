@@ -17,7 +17,7 @@
 //   degree <= S/64       a warp per vertex, table of S/32 slots
 //   degree <= S/16       128 threads per vertex, table of S/8 slots
 //   degree <= S/8        256 threads per vertex, table of S/4 slots
-//   larger               the CTA per vertex, table of S slots at load <= 2/3
+//   larger               the CTA per vertex, table of S slots at load <= 7/8
 // The tables are nested slices of one shared-memory region (a warp's slice
 // lies in its group's, a group's in the CTA's) and every vertex leaves its
 // slots empty, so a group moves on to the next kind of work without a CTA

@@ -14,8 +14,9 @@ constexpr unsigned kBarrierSpins = 1u << 24;
 // warp steps of a tile task in flight at once: SBM runs of 4.0 M entries took
 // 9.6 ms of kernel time with 1, 6.2 ms with 2 and 6.2 ms with 4 (spills)
 constexpr int kTileU = 2;
-// largest number of distinct communities a vertex may see: 2/3 of the CTA's table
-constexpr uint32_t kResidentCapacity = (1u << kResidentMaxBits) / 3 * 2;
+// largest number of distinct communities a vertex may see: 7/8 of the CTA's table (few vertices
+// are that large; the probes of a table filled so far cost less than leaving the level)
+constexpr uint32_t kResidentCapacity = (1u << kResidentMaxBits) / 8 * 7;
 
 // log2 of the slots of a CTA's table for a level of that largest degree (or
 // number of communities a vertex can see): as small as the level allows, since

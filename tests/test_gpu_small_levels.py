@@ -38,3 +38,37 @@ def test_coarsen_sizes(O, ctx, pairs, kind):
         np.testing.assert_allclose(wts, h.weight_array(), rtol=1e-12)
     else:
         assert (wts == h.weight_array()).all()
+
+
+@pytest.mark.parametrize("kind", ["unit", "int", "real"])
+@pytest.mark.parametrize("n,pairs", [(2, 1), (5, 6), (300, 1000), (1500, 4095), (1500, 4096), (1500, 4097),
+                                     (8191, 2000), (8192, 2000), (8193, 2000), (90, 3900)])
+def test_small_runs(O, ctx, n, pairs, kind):
+    """Runs whose levels lie on both sides of the one-block step from level to
+    level (8,192 vertices or entries): the oracle's run, and every level's
+    graph the oracle's coarsening of the level before."""
+    rng = np.random.default_rng(n + pairs)
+    key = np.unique(rng.integers(0, n * (n - 1) // 2, 4 * pairs))[:]
+    key = rng.permutation(key)[:pairs]
+    hi = ((1 + np.sqrt(1 + 8 * key.astype(np.float64))) // 2).astype(np.int64)
+    hi -= hi * (hi - 1) // 2 > key
+    lo = key - hi * (hi - 1) // 2
+    w = None if kind == "unit" else rng.integers(1, 9, len(key)).astype(np.float64) if kind == "int" else rng.random(len(key)) + 0.5
+    g = O.csr_from_pairs(n, lo, hi, w)
+    a = ctx.graph_from_csr(g.n, g.offsets, g.cols, g.weights).louvain(keep_levels=2)
+    cur = g
+    for lvl, (off, cols, wts) in enumerate(a["level_csr"]):
+        assert (off == cur.offsets).all() and (cols == cur.cols).all()
+        if kind == "real":  # sums of at most a few thousand doubles a level
+            np.testing.assert_allclose(wts, cur.weight_array(), rtol=1e-11)
+        else:
+            assert (wts == cur.weight_array()).all()
+        if lvl + 1 < len(a["level_csr"]):
+            _, cur, _ = O.coarsen(cur, a["level_maps"][lvl])
+    b = O.louvain(g)
+    if kind == "real":
+        assert abs(a["modularity"] - b["modularity"]) < 1e-3
+        assert abs(O.modularity(g, a["assignment"]) - a["modularity"]) < 1e-9
+    else:
+        assert (a["level_sizes"] == b["level_sizes"]).all() and (a["trace"] == b["trace"]).all()
+        assert (a["assignment"] == b["assignment"]).all()
