@@ -178,12 +178,13 @@ mg_status mg_local_move(mg_graph *g, int version, int up, int precision, const u
  * Work is queued on `stream` (a cudaStream_t, NULL = default stream); the call
  * waits for the stream once, to read the graph's maximum degree, so it must
  * not be called while that stream is being captured into a CUDA graph.
- * Scratch: the per-block hash tables live in one static 16 MiB device array
- * that every GPU loading the library holds until exit; each vertex uses a
- * table sized by its own degree.  A graph whose maximum degree needs a table
- * beyond it (a degree above 524,287) is rejected with MG_ERR_UNSUPPORTED.
- * The first call on a device looks up that array's device address (a
- * one-time set-up per device).  All calls share the array and clear it on
+ * Scratch: vertices of up to 10,922 edges use shared-memory tables; the tables
+ * of larger ones live in one static 16 MiB device array that every GPU loading
+ * the library holds until exit.  Each vertex uses a table sized by its own
+ * degree.  A graph whose maximum degree needs a table beyond the array (a degree
+ * above 524,287) is rejected with MG_ERR_UNSUPPORTED.
+ * The first call on a device looks up that array's device address and sets the
+ * kernels' shared-memory limits (a one-time set-up per device).  All calls share the array and clear it on
  * entry, so calls that overlap on the GPU race with each other.  Errors are
  * reported by mg_last_error(NULL). */
 mg_status mg_local_move_noalloc(uint32_t n, const uint32_t *d_offsets, const uint32_t *d_cols,
@@ -226,7 +227,8 @@ typedef struct {
     uint64_t phase0_edges_swept;
     double phase0_seconds;
     uint64_t distinct_pairs; /* sum over sweeps of the candidate pairs */
-    double seconds_sweep_kernels; /* device time of the local-move kernels alone */
+    double seconds_sweep_kernels; /* device time of the local-move kernels alone (levels that one resident
+                                     kernel iterates: that kernel, sigma updates included) */
     double sweep_bytes;      /* algorithmic bytes of those sweeps: 12E + 24V + 8D each */
     uint64_t kernel_launches; /* engine kernels launched during the run */
     uint64_t sweeps;         /* edge passes run (iterations + one per phase) */
@@ -272,7 +274,11 @@ mg_status mg_result_destroy(mg_result *r);
  * is not yet in the context's table, and the fastest is stored (keyed by weight
  * kind, precision, version, single / batched sweep, class and class size) and
  * reused.  MG_TUNE_OFF uses the built-in shapes, MG_TUNE_CACHED the table
- * without timing anything new, MG_TUNE_ON (default) also fills it. */
+ * without timing anything new, MG_TUNE_ON (default) also fills it.  With
+ * MG_TUNE_ON and the default sweep policy, levels of up to 20 M entries and
+ * batches of graphs that spread evenly over the SMs run in resident kernels
+ * (all iterations in one launch), which have no shapes to tune; the other modes
+ * and every forced sweep option use the class kernels throughout. */
 enum { MG_TUNE_OFF = 0, MG_TUNE_CACHED = 1, MG_TUNE_ON = 2 };
 mg_status mg_tune_mode(mg_ctx *ctx, int mode);
 /* The table as text, one entry per line:

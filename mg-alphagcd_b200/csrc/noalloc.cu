@@ -202,15 +202,16 @@ __device__ __forceinline__ void nb_vertex(const NoAllocArgs &A, uint32_t v, uint
     __syncwarp(lanes);  // the table is empty before the next vertex
 }
 
-// Degrees up to kWarpDeg: a warp takes 32 consecutive vertices, first those of
-// at most kLaneDeg edges, four at a time by 8 lanes, then the others.
+// Degrees up to kWarpDeg: a warp takes `per` consecutive vertices (4 to 32: as
+// many as leave every warp of the device some), first those of at most kLaneDeg
+// edges, four at a time by 8 lanes, then the others.
 // 4 blocks of 256 threads per SM (48 KB of tables each).
 constexpr uint32_t kLaneDeg = 32, kWarpDeg = 256, kGroupDeg = 2048, kCtaDeg = 10922;
 constexpr int kWarpBits = 9, kGroupBits = 12, kCtaBits = 14;
 constexpr int kCtaThreads = 1024;
 
 template <bool UNIT>
-__global__ void __launch_bounds__(kNoAllocThreads, 4) noalloc_warp_kernel(NoAllocArgs A) {
+__global__ void __launch_bounds__(kNoAllocThreads, 4) noalloc_warp_kernel(NoAllocArgs A, uint32_t per) {
     using V = NbVal<UNIT>;
     constexpr uint32_t S = 1u << kWarpBits;
     extern __shared__ __align__(16) unsigned char nb_smem[];
@@ -223,13 +224,15 @@ __global__ void __launch_bounds__(kNoAllocThreads, 4) noalloc_warp_kernel(NoAllo
     }
     __syncwarp();
     const uint32_t tile = lane / 8, lanes = 0xffu << (8 * tile);
-    const uint64_t step = (uint64_t)gridDim.x * kNoAllocThreads;
-    for (uint64_t v0 = (uint64_t)blockIdx.x * kNoAllocThreads + 32 * warp; v0 < A.n; v0 += step) {
+    constexpr uint32_t kWarps = kNoAllocThreads / 32;
+    const uint64_t step = (uint64_t)gridDim.x * kWarps * per;
+    for (uint64_t v0 = ((uint64_t)blockIdx.x * kWarps + warp) * per; v0 < A.n; v0 += step) {
         const uint64_t v = v0 + lane;
-        const uint32_t lo = v < A.n ? A.off[v] : 0u, hi = v < A.n ? A.off[v + 1] : 0u;
+        const bool mine = lane < per && v < A.n;
+        const uint32_t lo = mine ? A.off[v] : 0u, hi = mine ? A.off[v + 1] : 0u;
         const uint32_t d = hi - lo;
         // one tile's slice: a quarter of the warp's
-        for (uint32_t r = 0; r < 32; r += 4) {
+        for (uint32_t r = 0; r < per; r += 4) {
             const uint32_t q = r + tile;
             const uint32_t vd = __shfl_sync(0xffffffffu, d, q), vlo = __shfl_sync(0xffffffffu, lo, q);
             if (v0 + q < A.n && vd <= kLaneDeg)
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kNoAllocThreads, 4) noalloc_warp_kernel(NoAllo
                                    vals + tile * (S / 4), kWarpBits - 2);
             __syncwarp();
         }
-        uint32_t rest = __ballot_sync(0xffffffffu, v < A.n && d > kLaneDeg && d <= kWarpDeg);
+        uint32_t rest = __ballot_sync(0xffffffffu, mine && d > kLaneDeg && d <= kWarpDeg);
         for (; rest; rest &= rest - 1) {
             const uint32_t q = __ffs(rest) - 1;
             const uint32_t vd = __shfl_sync(0xffffffffu, d, q), vlo = __shfl_sync(0xffffffffu, lo, q);
@@ -290,14 +293,14 @@ __device__ __forceinline__ void nb_cta_vertex(const NoAllocArgs &A, uint32_t v, 
     __syncthreads();  // the table is empty, red_* are read
 }
 
-// The vertices of degrees in (dmin, dmax], a CTA each.  A CTA looks at NT
-// vertices at a time, eight consecutive ones (a sector of offsets) from each
-// of NT / 8 places spread over the ids, so that hubs with neighbouring ids
-// fall to different CTAs.  GLOBAL: the tables are the CTA's part of the scratch
+// The vertices of degrees in (dmin, dmax], a CTA each.  A CTA looks at `span`
+// vertices at a time (at most NT), eight consecutive ones (a sector of offsets)
+// from each of span / 8 places spread over the ids, so that hubs with
+// neighbouring ids fall to different CTAs.  GLOBAL: the tables are the CTA's part of the scratch
 // array (cleared by the host), else shared memory.
 template <int NT, bool UNIT, bool GLOBAL>
 __global__ void __launch_bounds__(NT) noalloc_cta_kernel(NoAllocArgs A, uint32_t dmin, uint32_t dmax, int most,
-                                                         uint32_t *tkeys, double *tvals) {
+                                                         uint32_t span, uint32_t *tkeys, double *tvals) {
     using V = NbVal<UNIT>;
     extern __shared__ __align__(16) unsigned char nb_smem[];
     __shared__ double red_g[NT / 32];
@@ -312,12 +315,12 @@ __global__ void __launch_bounds__(NT) noalloc_cta_kernel(NoAllocArgs A, uint32_t
             vals[s] = V(0);
         }
     }
-    const uint32_t eights = (uint32_t)(((uint64_t)A.n + 7) / 8), rounds = (eights + NT / 8 - 1) / (NT / 8);
+    const uint32_t eights = (uint32_t)(((uint64_t)A.n + 7) / 8), rounds = (eights + span / 8 - 1) / (span / 8);
     for (uint32_t r = blockIdx.x; r < rounds; r += gridDim.x) {
         if (threadIdx.x == 0) count = 0;
         __syncthreads();
         const uint64_t v = ((uint64_t)r + (uint64_t)(threadIdx.x / 8) * rounds) * 8 + threadIdx.x % 8;
-        if (v < A.n) {
+        if (threadIdx.x < span && v < A.n) {
             const uint32_t d = A.off[v + 1] - A.off[v];
             if (d > dmin && d <= dmax) list[atomicAdd(&count, 1u)] = (uint32_t)v;
         }
@@ -353,24 +356,38 @@ cudaError_t nb_set_limits() {
 template <bool UNIT>
 void nb_launch(const NoAllocArgs &A, uint32_t maxdeg, uint32_t blocks, uint32_t tsize, uint32_t *tkeys, double *tvals,
                cudaStream_t s) {
+    // vertices per CTA and round: as many as leave `ctas` CTAs some
+    auto span_for = [&](uint32_t nt, uint64_t ctas) {
+        uint32_t span = nt;
+        while (span > 8 && A.n / span < ctas) span /= 2;
+        return span;
+    };
+    auto grid_for = [&](uint32_t span, uint64_t ctas) {
+        return (unsigned)std::min<uint64_t>(ctas, ceil_div(ceil_div(A.n, 8), span / 8));
+    };
     if (maxdeg > kCtaDeg) {
         // the scratch keeps the previous call's contents: clear the tables
         noalloc_clear_kernel<<<148 * 4, 256, 0, s>>>(tkeys, tvals, (size_t)blocks * tsize);
-        noalloc_cta_kernel<kCtaThreads, UNIT, true>
-            <<<blocks, kCtaThreads, 0, s>>>(A, kCtaDeg, 0xFFFFFFFFu, 31 - __builtin_clz(tsize), tkeys, tvals);
+        noalloc_cta_kernel<kCtaThreads, UNIT, true><<<blocks, kCtaThreads, 0, s>>>(
+            A, kCtaDeg, 0xFFFFFFFFu, 31 - __builtin_clz(tsize), span_for(kCtaThreads, blocks), tkeys, tvals);
     }
-    const uint32_t eights = (uint32_t)ceil_div(A.n, 8);
-    if (maxdeg > kGroupDeg)
+    if (maxdeg > kGroupDeg) {
+        const uint32_t span = span_for(kCtaThreads, 148);
         noalloc_cta_kernel<kCtaThreads, UNIT, false>
-            <<<std::min<uint32_t>(148, (eights + kCtaThreads / 8 - 1) / (kCtaThreads / 8)), kCtaThreads,
-               nb_smem_bytes<UNIT>(kCtaBits, 1), s>>>(A, kGroupDeg, kCtaDeg, kCtaBits, nullptr, nullptr);
-    if (maxdeg > kWarpDeg)
+            <<<grid_for(span, 148), kCtaThreads, nb_smem_bytes<UNIT>(kCtaBits, 1), s>>>(A, kGroupDeg, kCtaDeg, kCtaBits,
+                                                                                        span, nullptr, nullptr);
+    }
+    if (maxdeg > kWarpDeg) {
+        const uint32_t span = span_for(kNoAllocThreads, 148 * 4);
         noalloc_cta_kernel<kNoAllocThreads, UNIT, false>
-            <<<std::min<uint32_t>(148 * 4, (eights + kNoAllocThreads / 8 - 1) / (kNoAllocThreads / 8)), kNoAllocThreads,
-               nb_smem_bytes<UNIT>(kGroupBits, 1), s>>>(A, kWarpDeg, kGroupDeg, kGroupBits, nullptr, nullptr);
-    noalloc_warp_kernel<UNIT>
-        <<<(unsigned)std::min<uint64_t>(148 * 4, ceil_div(A.n, kNoAllocThreads)), kNoAllocThreads,
-           nb_smem_bytes<UNIT>(kWarpBits, kNoAllocThreads / 32), s>>>(A);
+            <<<grid_for(span, 148 * 4), kNoAllocThreads, nb_smem_bytes<UNIT>(kGroupBits, 1), s>>>(
+                A, kWarpDeg, kGroupDeg, kGroupBits, span, nullptr, nullptr);
+    }
+    constexpr uint64_t kWarps = kNoAllocThreads / 32;
+    uint32_t per = 32;
+    while (per > 4 && A.n / per < 148 * 4 * kWarps) per /= 2;
+    noalloc_warp_kernel<UNIT><<<(unsigned)std::min<uint64_t>(148 * 4, ceil_div(A.n, per * kWarps)), kNoAllocThreads,
+                                nb_smem_bytes<UNIT>(kWarpBits, kNoAllocThreads / 32), s>>>(A, per);
 }
 
 mg_status noalloc_fail(mg_status st, const std::string &msg) {
