@@ -743,10 +743,11 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
         phase_init_kernel<<<(unsigned)ceil_div(G, 256), 256, 0, s>>>(alive_d, G, W.gword.get(), W.sums.get(),
                                                                      W.loops.get(), ctrl);
         MG_LAUNCH_CHECK();
-        level_init(cur, k, sigma, C[0], s);
+        level_init(cur, k, sigma, C[0], s, false);
         if (phase > 0)  // (level 0: the batch's own entry offsets)
             MG_CUDA(cudaMemcpyAsync(hnnz.data(), W.gnnz.get(), sizeof(uint32_t) * G, cudaMemcpyDeviceToHost, s));
         move_prepare_level(cur, mlv, ctx->mws, s);
+        level_init_long(cur, mlv, k, sigma, s);
         MG_CUDA(cudaStreamSynchronize(s));
         sweep_reset_acc(ctx->mws, s);
         std::vector<uint32_t> order;

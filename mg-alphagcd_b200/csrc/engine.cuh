@@ -308,8 +308,12 @@ void sigma_sumsq(const double *sigma, uint32_t n, int integral, MoveWorkspace &w
 // sigma += k moved from P[v] to N[v]; counts moved vertices into ws.acc
 void sigma_update(const uint32_t *P, const uint32_t *N, const double *k, double *sigma, uint32_t n,
                   MoveWorkspace &ws, cudaStream_t s);
-// k_i = row sums; sigma = k; C = identity
-void level_init(const GraphView &g, double *k, double *sigma, uint32_t *C, cudaStream_t s);
+// k_i = row sums; sigma = k; C = identity.  Without long_rows the weights of the
+// heavy classes' vertices (rows above kLongRow entries) are left to
+// level_init_long, which takes their list from the prepared level.
+constexpr uint32_t kLongRow = 4096;
+void level_init(const GraphView &g, double *k, double *sigma, uint32_t *C, cudaStream_t s, bool long_rows = true);
+void level_init_long(const GraphView &g, const MoveLevel &lvl, double *k, double *sigma, cudaStream_t s);
 // The sums of the modularity of C into ws.acc (zeroed by the caller): one pass
 // over the edges, without the candidate tables of a sweep.  k, sigma and
 // scratch are work buffers of n entries.

@@ -135,8 +135,9 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         double phase_lm = 0;
         Timer tp(ctx->ev[0], ctx->ev[1], s);
         if (!prepared) {
-            level_init(cur, k, sigma, C[0], s);
+            level_init(cur, k, sigma, C[0], s, false);
             move_prepare_level(cur, mlv, ctx->mws, s);
+            level_init_long(cur, mlv, k, sigma, s);
         }
         prepared = false;
         bool resident = false;
