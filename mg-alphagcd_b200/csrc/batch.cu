@@ -508,7 +508,7 @@ __global__ void class_starts_kernel(const uint32_t *perm, Idx19 off, const uint3
 int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vector<uint32_t> &alive,
                   const std::vector<uint64_t> &load, uint32_t most_vertices) {
     constexpr double kSmRate = 440, kSweepMin = 8, kClassRate = 46e3, kClassSweep = 120;
-    if (ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
+    if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
     if (std::min(lvl.bins.max_degree, most_vertices) > lmr::kResidentCapacity) return 0;
     double total = 0;
     for (uint32_t g : alive) total += (double)load[g];

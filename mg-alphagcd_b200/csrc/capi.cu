@@ -24,6 +24,10 @@ mg_status fail(mg_ctx *ctx, mg_status st, const std::string &msg) {
 
 template <class F>
 mg_status guarded(mg_ctx *ctx, F &&f) {
+    struct Pool {  // allocations of this entry point may draw on the context's pool
+        explicit Pool(BufPool *p) { t_pool = p; }
+        ~Pool() { t_pool = nullptr; }
+    } pool(ctx ? &ctx->pool : nullptr);
     try {
         if (ctx) MG_CUDA(cudaSetDevice(ctx->device));
         f();
@@ -59,6 +63,7 @@ mg_ctx::~mg_ctx() {
 
 namespace mg {
 thread_local unsigned long long g_kernel_launches = 0;
+thread_local BufPool *t_pool = nullptr;
 
 static std::atomic<long long> g_alloc_fault_countdown{0};  // 0: disarmed
 

@@ -124,6 +124,9 @@ private:
     size_t total_ = 0;
 };
 
+// The pool of the context whose entry point this thread is in (null: none).
+extern thread_local BufPool *t_pool;
+
 // Grow-only device allocation owned by the engine (cudaMalloc on growth only),
 // from and back to a pool where it has one.
 template <class T>
@@ -144,24 +147,32 @@ struct DBuf {
     }
     T *ensure(size_t n) {
         if (n > cap) {
+            // a large buffer that has to grow a little (the next graph is of
+            // about the same size) grows by a sixteenth more, memory permitting,
+            // so that not every new largest graph reallocates the workspace
+            const bool again = cap * sizeof(T) >= kSlackFrom && n < cap + cap / 4;
             release();
-            size_t want = n < 16 ? 16 : n;
+            const size_t want = n < 16 ? 16 : n, roomy = again ? want + want / 16 : want;
             if (alloc_fault_due()) throw Error(MG_ERR_OOM, "device allocation failed (injected by mg_test_fail_allocation)");
             size_t got = 0;
             if (pool && (p = (T *)pool->take(want * sizeof(T), got))) {
                 cap = got / sizeof(T);
                 return p;
             }
-            if (pool && cudaMalloc(&p, want * sizeof(T)) != cudaSuccess) {
-                cudaGetLastError();  // once more with what the pool holds given back
-                p = nullptr;
-                pool->trim();
+            if (cudaMalloc(&p, roomy * sizeof(T)) == cudaSuccess) {
+                cap = roomy;
+                return p;
             }
-            if (!p) MG_CUDA(cudaMalloc(&p, want * sizeof(T)));
+            // once more as asked, with what the context's pool holds given back
+            cudaGetLastError();
+            p = nullptr;
+            if (t_pool) t_pool->trim();
+            MG_CUDA(cudaMalloc(&p, want * sizeof(T)));
             cap = want;
         }
         return p;
     }
+    static constexpr size_t kSlackFrom = 1u << 20;  // bytes
     T *get() const { return p; }
 };
 

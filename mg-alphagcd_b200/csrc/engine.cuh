@@ -194,7 +194,10 @@ struct MoveWorkspace {
     // the kernels it names, also on levels that the resident kernels would run
     // (nor do these run when the caller fixes the shapes, MG_TUNE_OFF / CACHED)
     bool forced_policy = false;
-    DBuf<unsigned char> resident;  // resident level kernel: state, sums, counters, barrier
+    // the resident kernels (blocks that take a whole SM) may run; not where
+    // other contexts' work shares the device (a server with several slots)
+    bool resident = true;
+    DBuf<unsigned char> res_block;  // resident level kernel: state, sums, counters, barrier
     void *h_resident = nullptr;    // pinned image of them
     DBuf<SmallInfo> small;         // counts of a small level
     PrimWorkspace prim;

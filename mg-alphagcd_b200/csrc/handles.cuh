@@ -40,11 +40,12 @@ public:
         return *this;
     }
     ~HostIds() { release(); }
-    // n uninitialised ids; does nothing when they are there already
+    // n uninitialised ids (plain memory without a spare buffer); does nothing
+    // when they are there already
     void ensure(size_t n, const std::shared_ptr<PinnedSpare> &spare) {
         if (p_ && n_ == n) return;
         release();
-        if (n >= kPinnedFrom && n <= kPinnedIds) {
+        if (spare && n >= kPinnedFrom && n <= kPinnedIds) {
             std::lock_guard<std::mutex> lk(spare->mu);
             if (!lent_ok(*spare, n)) return plain(n);
             p_ = spare->p;

@@ -24,7 +24,7 @@ struct ResidentBlock {
 }  // namespace
 
 bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws) {
-    if (ws.forced_policy || ws.tune.mode != MG_TUNE_ON || g.n == 0 || g.nnz > kResidentMaxEntries) return false;
+    if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON || g.n == 0 || g.nnz > kResidentMaxEntries) return false;
     return std::min(lvl.bins.max_degree, g.n) <= kResidentCapacity;
 }
 
@@ -37,7 +37,7 @@ void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const S
         MG_CUDA(cudaMallocHost(&ws.h_resident, sizeof(ResidentBlock)));
         hb = (ResidentBlock *)ws.h_resident;
     }
-    ResidentBlock *db = (ResidentBlock *)ws.resident.ensure(sizeof(ResidentBlock));
+    ResidentBlock *db = (ResidentBlock *)ws.res_block.ensure(sizeof(ResidentBlock));
     ResidentArgs A = {};
     A.col = g.col;
     A.w = g.w;

@@ -198,6 +198,14 @@ void worker_main(mg_server *S) {
         return;
     }
     std::unique_ptr<mg_batch> b(new mg_batch());
+    // several slots share the device: a cluster of whole-SM blocks would wait
+    // behind the other slots' small blocks, which fill every SM as it frees up
+    // (6 req/s: p50 latency 0.019 -> 0.046 s, p99 0.66 -> 1.8 s), and making or
+    // freeing page-locked memory would wait for the other slots' work
+    if (S->opts.slots > 1) {
+        ctx->mws.resident = false;
+        ctx->spare.reset();
+    }
     b->ctx = ctx;
     b->u.ctx = ctx;
     while (true) {
