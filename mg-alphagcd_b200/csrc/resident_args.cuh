@@ -12,7 +12,8 @@ constexpr int kResidentIters = 48;     // iterations of one launch (the host lau
 constexpr int kResidentMaxBits = 14;   // slots of a CTA's table: 2^14 (9 or 13 bytes each)
 constexpr unsigned kBarrierSpins = 1u << 24;
 // warp steps of a tile task in flight at once: SBM runs of 4.0 M entries took
-// 9.6 ms of kernel time with 1, 6.2 ms with 2 and 6.2 ms with 4 (spills)
+// 5.8 ms of kernel time with 1, 5.0 ms with 2, 5.6 ms with 3 and 5.3 ms with 4
+// (spills)
 constexpr int kTileU = 2;
 // largest number of distinct communities a vertex may see: 7/8 of the CTA's table (few vertices
 // are that large; the probes of a table filled so far cost less than leaving the level)
