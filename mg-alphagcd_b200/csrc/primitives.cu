@@ -144,7 +144,7 @@ static void scan_level(const T *in, T *out, size_t n, T *d_total, cudaStream_t s
         if (d_total) MG_CUDA(cudaMemsetAsync(d_total, 0, sizeof(T), s));
         return;
     }
-    if (n <= kScanOne) {
+    if (ws.one_block && n <= kScanOne) {
         scan_one_kernel<T><<<1, kScanOneThreads, 0, s>>>(in, out, (uint32_t)n, d_total);
         MG_LAUNCH_CHECK();
         return;
@@ -399,7 +399,7 @@ bool radix_sort(uint64_t *keys, V *vals, uint64_t *keys_alt, V *vals_alt, size_t
                 cudaStream_t s, PrimWorkspace &ws, int lo_bit) {
     if (n <= 1 || bits <= lo_bit) return false;
     MG_CHECK(n < 0xFFFFFFFFull, MG_ERR_UNSUPPORTED, "radix_sort: more than 2^32-1 keys");
-    if (n <= kRsOne) {
+    if (ws.one_block && n <= kRsOne) {
         MG_CUDA(cudaFuncSetAttribute(rs_one_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)rs_one_smem<V>()));
         rs_one_kernel<V><<<1, kRsOneThreads, rs_one_smem<V>(), s>>>(keys, vals, keys_alt, vals_alt, (uint32_t)n,

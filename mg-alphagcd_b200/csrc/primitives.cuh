@@ -17,6 +17,8 @@ struct PrimWorkspace {
     DBuf<uint64_t> scan_a, scan_b, scan_c;  // block sums of the scan levels
     DBuf<uint32_t> hist;                    // radix tile histograms
     DBuf<uint32_t> bins;                    // degree-bin block counts
+    bool one_block = true;                  // small scans and sorts as one block of 1,024 threads (not
+                                            // where other contexts' small blocks fill the device)
     uint32_t *h_small = nullptr;            // pinned words for counts read back
     uint32_t *pinned();                     // kPinnedWords of them
     ~PrimWorkspace();

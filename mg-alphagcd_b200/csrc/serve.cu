@@ -204,6 +204,7 @@ void worker_main(mg_server *S) {
     // freeing page-locked memory would wait for the other slots' work
     if (S->opts.slots > 1) {
         ctx->mws.resident = false;
+        ctx->mws.prim.one_block = ctx->cws.prim.one_block = false;
         ctx->spare.reset();
     }
     b->ctx = ctx;
