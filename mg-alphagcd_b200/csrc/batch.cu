@@ -495,40 +495,14 @@ __global__ void class_starts_kernel(const uint32_t *perm, Idx19 off, const uint3
     out[i] = lo;
 }
 
-// CTAs per graph for a phase of the resident kernel, 0 when the class kernels
-// serve it better.  Both are estimated per sweep: a CTA sweeps kSmRate entries
-// per microsecond and a sweep takes kSweepMin at least; clusters take the graphs
-// in turn, largest first, so a phase ends near the larger of the mean load of a
-// cluster and the largest graph's (a third of the smaller is added for graphs that
-// take more iterations than others).  The class kernels sweep kClassRate
-// entries per microsecond over all graphs and pay kClassSweep per sweep for
-// launches and the per-graph sums.  (One graph among many that is too large for
-// a cluster, or a vertex of more communities than a CTA's table holds, sends
-// the phase there.)
 int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vector<uint32_t> &alive,
-                  const std::vector<uint64_t> &load, uint32_t most_vertices) {
-    constexpr double kSmRate = 440, kSweepMin = 8, kClassRate = 46e3, kClassSweep = 120;
+                  const std::vector<uint64_t> &load, uint32_t most_vertices, int wk, int integral) {
     if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
     if (std::min(lvl.bins.max_degree, most_vertices) > lmr::kResidentCapacity) return 0;
-    double total = 0;
-    for (uint32_t g : alive) total += (double)load[g];
-    double best = total / kClassRate + kClassSweep;
-    int ctas = 0;
-    for (int cs = 1; cs <= 8; cs *= 2) {
-        double sum = 0, most = 0;
-        for (uint32_t g : alive) {
-            const double t = std::max(kSweepMin, (double)load[g] / (cs * kSmRate));
-            sum += t;
-            most = std::max(most, t);
-        }
-        const double clusters = kNumSMs / cs;
-        const double mean = sum / clusters, est = std::max(most, mean) + 0.35 * std::min(most, mean);
-        if (est < best) {
-            best = est;
-            ctas = cs;
-        }
-    }
-    return ctas;
+    std::vector<uint64_t> l;
+    l.reserve(alive.size());
+    for (uint32_t g : alive) l.push_back(load[g]);
+    return resident_team(l.data(), (uint32_t)l.size(), !integral ? 2 : wk == WK_UNIT ? 0 : 1, kNumSMs);
 }
 
 void launch_batch(const lmr::ResidentBatchArgs &A, int wk, const SweepParams &p, int ctas, unsigned most,
@@ -618,6 +592,53 @@ void resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLeve
 }
 
 }  // namespace
+
+// Both forms are estimated per sweep, in microseconds.  A CTA sweeps `rate`
+// entries per microsecond and a sweep takes kSweepMin at least; clusters take the
+// graphs in turn, largest first, so a phase ends near the larger of the mean load
+// of a cluster and the largest graph's, plus a part of the smaller for graphs that
+// take more iterations than others.  The class kernels sweep 46,000 to 50,000
+// entries per microsecond over all graphs and pay 120 to 200 us per sweep for
+// launches and the per-graph sums.
+// With weights a CTA is slower (table sums) and iteration counts spread further,
+// so a large graph with many iterations holds its cluster while the others are
+// done, which the class kernels spread over the device: the team has to win with
+// that graph's load taken 1.4 times as well.
+// Measured on the 601 phases of SBM batches (12 to 256 graphs of 1,000 to 200,000
+// vertices, both versions, with and without hubs of 5,000 edges), each timed with
+// the class kernels and with teams of 1, 2, 4 and 8 CTAs.  Sums in ms by this rule /
+// with the best choice of each phase / with the class kernels alone: unit weights
+// 489 / 470 / 603, integer weights 625 / 589 / 721, real weights 1,979 / 1,921 /
+// 2,164, and no phase above 0.5 ms longer than with the class kernels; without the
+// second condition real weights took 2,402, single phases up to 1.9 times the
+// class kernels.
+int resident_team(const uint64_t *load, uint32_t graphs, int weights, int sms) {
+    constexpr double kSweepMin = 8;
+    double total = 0;
+    for (uint32_t i = 0; i < graphs; i++) total += (double)load[i];
+    auto team = [&](int cs, double rate, double risk, double part) {
+        double sum = 0, most = 0;
+        for (uint32_t i = 0; i < graphs; i++) {
+            const double t = std::max(kSweepMin, (double)load[i] / (cs * rate));
+            sum += t;
+            most = std::max(most, t);
+        }
+        const double mean = sum * cs / sms, last = risk * most;
+        return std::max(last, mean) + part * std::min(last, mean);
+    };
+    auto classes = [&](double rate, double launches) { return total / (rate / kNumSMs * sms) + launches; };
+    double best = classes(46e3, 120);
+    int ctas = 0;
+    for (int cs = 1; cs <= 8; cs *= 2) {
+        const double est = team(cs, 440, 1, 0.35);
+        if (est < best) {
+            best = est;
+            ctas = cs;
+        }
+    }
+    if (ctas && weights && team(ctas, weights == 1 ? 360 : 320, 1.4, 0.3) >= classes(50e3, 200)) ctas = 0;
+    return ctas;
+}
 
 void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &res, const GraphDoneFn *done) {
     mg_ctx *ctx = b->ctx;
@@ -759,7 +780,7 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
             most_vertices = std::max(most_vertices, ng);
             load[g] = hnnz[g] + 4ull * ng;
         }
-        const int ctas = resident_ctas(ctx->mws, mlv, order, load, most_vertices);
+        const int ctas = resident_ctas(ctx->mws, mlv, order, load, most_vertices, cur.wk, integral);
         if (ctas > 0) {
             std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return load[x] > load[y]; });
             resident_phase(ctx, b, cur, mlv, sp, thr, goff, order, ctas, S, s);

@@ -612,6 +612,12 @@ mg_status mg_test_fail_allocation(uint64_t nth, uint64_t *pending) {
     return MG_OK;
 }
 
+mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int weights, int sms, int *ctas) {
+    if (!ctas || (graphs && !loads) || weights < 0 || weights > 2 || sms < 1) return MG_ERR_INVALID;
+    *ctas = resident_team(loads, graphs, weights, sms);
+    return MG_OK;
+}
+
 mg_status mg_sweep_options(mg_ctx *ctx, const mg_sweep_opts *opts) {
     if (!ctx) return MG_ERR_INVALID;
     const int fill = opts ? opts->cluster_fill : MG_FILL_AUTO;

@@ -1,0 +1,46 @@
+"""The rules that choose between the resident and the class kernels, on the
+CPU.  The measured times (ms of a phase on a B200, by CTAs per graph, 0 = the
+class kernels) are of SBM batches whose graphs' sizes are log-uniform: the
+choice is never more than 3 % slower than the class kernels, which served every
+batch before there was a choice."""
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+UNIT, INTEGER, REAL = 0, 1, 2
+
+
+def _team(mg, loads, weights, sms=148):
+    a, out = np.ascontiguousarray(loads, np.uint64), ct.c_int(-1)
+    assert mg.lib().mg_test_batch_team(len(a), a.ctypes.data_as(ct.c_void_p), weights, sms, ct.byref(out)) == 0
+    return out.value
+
+
+@pytest.mark.parametrize("graphs,lo,hi,weights,ms", [
+    (200, 1000, 8000, UNIT, {0: 9.28, 1: 17.85, 2: 4.24, 4: 4.33, 8: 5.79}),
+    (200, 1000, 8000, INTEGER, {0: 10.78, 1: 16.73, 2: 6.71, 4: 6.11, 8: 7.60}),
+    (200, 1000, 8000, REAL, {0: 13.41, 1: 30.11, 2: 15.17, 4: 8.99, 8: 11.39}),
+    (48, 8000, 50000, UNIT, {0: 17.33, 1: 72.91, 2: 37.36, 4: 19.64, 8: 13.08}),
+    (48, 8000, 50000, REAL, {0: 30.86, 1: 413.69, 2: 210.41, 4: 109.75, 8: 57.66}),
+    (24, 30000, 60000, UNIT, {0: 17.31, 1: 92.17, 2: 47.67, 4: 24.45, 8: 14.96}),
+    (24, 30000, 60000, REAL, {0: 19.03, 1: 209.57, 2: 106.51, 4: 54.19, 8: 27.89}),
+    (96, 8000, 100000, INTEGER, {0: 67.61, 1: 671.0, 2: 338.11, 4: 172.36, 8: 90.94}),
+    (96, 8000, 100000, REAL, {0: 73.7, 1: 643.85, 2: 326.41, 4: 167.25, 8: 88.23}),
+    (256, 1000, 100000, REAL, {0: 119.43, 1: 1296.2, 2: 660.74, 4: 337.21, 8: 174.54}),
+])
+def test_batch_team(mg, graphs, lo, hi, weights, ms):
+    loads = np.geomspace(lo, hi, graphs) * 24  # 20 entries per vertex, and 4 per vertex
+    assert ms[_team(mg, loads, weights)] <= 1.03 * ms[0]
+
+
+def test_batch_team_bounds(mg):
+    assert _team(mg, [], UNIT) in (0, 1, 2, 4, 8)
+    for weights in (UNIT, INTEGER, REAL):
+        assert _team(mg, [2**40], weights) == 0  # one graph too large for a cluster
+        assert _team(mg, [20000] * 500, weights) in (1, 2, 4, 8)
+        for sms in (1, 7, 8, 20, 148):
+            assert _team(mg, [20000] * 50, weights, sms) in (0, 1, 2, 4, 8)
+    out = ct.c_int()
+    assert mg.lib().mg_test_batch_team(1, None, UNIT, 148, ct.byref(out)) != 0
+    assert mg.lib().mg_test_batch_team(0, None, 3, 148, ct.byref(out)) != 0
