@@ -336,8 +336,8 @@ mg_status mg_test_fail_allocation(uint64_t nth, uint64_t *pending);
 /* ---- dispatch rules (test hook, no GPU needed) ----------------------------------
  * CTAs per graph that a batch's phase takes in the resident kernel on a device
  * of `sms` SMs (1, 2, 4 or 8; 0: the class kernels), for graphs of the given
- * loads (entries + 4 * vertices).  weights: 0 unit, 1 integer, 2 real. */
-mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int weights, int sms, int *ctas);
+ * loads (entries + 4 * vertices) with integral or real weights. */
+mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int integral, int sms, int *ctas);
 
 /* ---- batched form --------------------------------------------------------------
  * No reference counterpart: the reference runs one graph per process.  A batch

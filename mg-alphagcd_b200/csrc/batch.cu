@@ -496,13 +496,13 @@ __global__ void class_starts_kernel(const uint32_t *perm, Idx19 off, const uint3
 }
 
 int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vector<uint32_t> &alive,
-                  const std::vector<uint64_t> &load, uint32_t most_vertices, int wk, int integral) {
+                  const std::vector<uint64_t> &load, uint32_t most_vertices, int integral) {
     if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
     if (std::min(lvl.bins.max_degree, most_vertices) > lmr::kResidentCapacity) return 0;
     std::vector<uint64_t> l;
     l.reserve(alive.size());
     for (uint32_t g : alive) l.push_back(load[g]);
-    return resident_team(l.data(), (uint32_t)l.size(), !integral ? 2 : wk == WK_UNIT ? 0 : 1, kNumSMs);
+    return resident_team(l.data(), (uint32_t)l.size(), !integral, kNumSMs);
 }
 
 void launch_batch(const lmr::ResidentBatchArgs &A, int wk, const SweepParams &p, int ctas, unsigned most,
@@ -597,22 +597,22 @@ void resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLeve
 // entries per microsecond and a sweep takes kSweepMin at least; clusters take the
 // graphs in turn, largest first, so a phase ends near the larger of the mean load
 // of a cluster and the largest graph's, plus a part of the smaller for graphs that
-// take more iterations than others.  The class kernels sweep 46,000 to 50,000
-// entries per microsecond over all graphs and pay 120 to 200 us per sweep for
-// launches and the per-graph sums.
-// With weights a CTA is slower (table sums) and iteration counts spread further,
-// so a large graph with many iterations holds its cluster while the others are
-// done, which the class kernels spread over the device: the team has to win with
-// that graph's load taken 1.4 times as well.
+// take more iterations than others.  The class kernels sweep 46,000 entries per
+// microsecond over all graphs and pay 120 us per sweep for launches and the
+// per-graph sums (220 with the sweeps of the last graphs alone).
+// With real weights a CTA is slower (its tables add doubles by compare-and-swap) and
+// iteration counts spread further, so a large graph with many iterations holds its
+// cluster while the others are done, which the class kernels spread over the
+// device: the team has to win at that rate with the graph's load taken 1.4 times.
 // Measured on the 601 phases of SBM batches (12 to 256 graphs of 1,000 to 200,000
 // vertices, both versions, with and without hubs of 5,000 edges), each timed with
 // the class kernels and with teams of 1, 2, 4 and 8 CTAs.  Sums in ms by this rule /
 // with the best choice of each phase / with the class kernels alone: unit weights
-// 489 / 470 / 603, integer weights 625 / 589 / 721, real weights 1,979 / 1,921 /
-// 2,164, and no phase above 0.5 ms longer than with the class kernels; without the
-// second condition real weights took 2,402, single phases up to 1.9 times the
-// class kernels.
-int resident_team(const uint64_t *load, uint32_t graphs, int weights, int sms) {
+// 490 / 470 / 603, integer weights 624 / 589 / 721, real weights 1,984 / 1,921 /
+// 2,164 (2,402 without the condition for them, single phases up to 1.9 times the
+// class kernels).  The same condition for integer weights gains on some phases what
+// it loses on others (625).
+int resident_team(const uint64_t *load, uint32_t graphs, int real, int sms) {
     constexpr double kSweepMin = 8;
     double total = 0;
     for (uint32_t i = 0; i < graphs; i++) total += (double)load[i];
@@ -636,7 +636,7 @@ int resident_team(const uint64_t *load, uint32_t graphs, int weights, int sms) {
             ctas = cs;
         }
     }
-    if (ctas && weights && team(ctas, weights == 1 ? 360 : 320, 1.4, 0.3) >= classes(50e3, 200)) ctas = 0;
+    if (ctas && real && team(ctas, 320, 1.4, 0.3) >= classes(46e3, 220)) ctas = 0;
     return ctas;
 }
 
@@ -780,7 +780,7 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
             most_vertices = std::max(most_vertices, ng);
             load[g] = hnnz[g] + 4ull * ng;
         }
-        const int ctas = resident_ctas(ctx->mws, mlv, order, load, most_vertices, cur.wk, integral);
+        const int ctas = resident_ctas(ctx->mws, mlv, order, load, most_vertices, integral);
         if (ctas > 0) {
             std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return load[x] > load[y]; });
             resident_phase(ctx, b, cur, mlv, sp, thr, goff, order, ctas, S, s);

@@ -612,9 +612,9 @@ mg_status mg_test_fail_allocation(uint64_t nth, uint64_t *pending) {
     return MG_OK;
 }
 
-mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int weights, int sms, int *ctas) {
-    if (!ctas || (graphs && !loads) || weights < 0 || weights > 2 || sms < 1) return MG_ERR_INVALID;
-    *ctas = resident_team(loads, graphs, weights, sms);
+mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int integral, int sms, int *ctas) {
+    if (!ctas || (graphs && !loads) || sms < 1) return MG_ERR_INVALID;
+    *ctas = resident_team(loads, graphs, !integral, sms);
     return MG_OK;
 }
 

@@ -345,8 +345,8 @@ void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const S
 // CTAs per graph (1, 2, 4, 8) for a phase of a batch in the resident kernel, 0
 // when the class kernels serve it better (one graph among many that is too large
 // for a cluster sends the phase there).  load: entries + 4 * vertices of every
-// graph still running; weights: 0 unit, 1 integer, 2 real; sms: SMs of the device.
-int resident_team(const uint64_t *load, uint32_t graphs, int weights, int sms);
+// graph still running; real: real weights; sms: SMs of the device.
+int resident_team(const uint64_t *load, uint32_t graphs, int real, int sms);
 
 // Coarsening.  out_off/out_col/out_w are resized as needed.
 struct CoarsenWorkspace {
