@@ -275,7 +275,8 @@ mg_status mg_result_destroy(mg_result *r);
  * kind, precision, version, single / batched sweep, class and class size) and
  * reused.  MG_TUNE_OFF uses the built-in shapes, MG_TUNE_CACHED the table
  * without timing anything new, MG_TUNE_ON (default) also fills it.  With
- * MG_TUNE_ON and the default sweep policy, levels of up to 20 M entries and
+ * MG_TUNE_ON and the default sweep policy, levels of up to 21 M entries (14.7 M with
+ * real weights; one vertex sees at most 14,336 communities) and
  * batches of graphs that spread evenly over the SMs run in resident kernels
  * (all iterations in one launch), which have no shapes to tune; the other modes
  * and every forced sweep option use the class kernels throughout. */
@@ -338,6 +339,9 @@ mg_status mg_test_fail_allocation(uint64_t nth, uint64_t *pending);
  * of `sms` SMs (1, 2, 4 or 8; 0: the class kernels), for graphs of the given
  * loads (entries + 4 * vertices) with integral or real weights. */
 mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int integral, int sms, int *ctas);
+/* *resident = 1 when a run's level of n vertices, nnz entries and that largest
+ * degree takes the resident kernel by default, 0 when the class kernels. */
+mg_status mg_test_level_resident(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral, int *resident);
 
 /* ---- batched form --------------------------------------------------------------
  * No reference counterpart: the reference runs one graph per process.  A batch

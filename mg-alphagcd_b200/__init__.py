@@ -123,7 +123,7 @@ EXPORTED = [
     "mg_tune_mode", "mg_tune_table", "mg_tune_save", "mg_tune_load", "mg_graph_generate_chunglu",
     "mg_graph_from_mtx_ex", "mg_csr_from_mtx", "mg_csr_info", "mg_csr_arrays", "mg_csr_free",
     "mg_result_level_map", "mg_result_level_csr", "mg_sweep_options", "mg_test_fail_allocation",
-    "mg_test_batch_team",
+    "mg_test_batch_team", "mg_test_level_resident",
 ]
 TUNE_OFF, TUNE_CACHED, TUNE_ON = 0, 1, 2
 FILL_AUTO, FILL_OWN, FILL_SPLIT = 0, 1, 2
@@ -194,6 +194,7 @@ def lib():
     L.mg_sweep_options.argtypes = [vp, ct.POINTER(_SweepOpts)]
     L.mg_test_fail_allocation.argtypes = [u64, ct.POINTER(u64)]
     L.mg_test_batch_team.argtypes = [u32, vp, i32, i32, ct.POINTER(i32)]
+    L.mg_test_level_resident.argtypes = [u32, u64, u32, i32, ct.POINTER(i32)]
     L.mg_tune_table.argtypes = [vp, ct.c_char_p, ct.c_size_t, ct.POINTER(ct.c_size_t)]
     L.mg_tune_save.argtypes = [vp, ct.c_char_p]
     L.mg_tune_load.argtypes = [vp, ct.c_char_p]

@@ -618,6 +618,12 @@ mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int integra
     return MG_OK;
 }
 
+mg_status mg_test_level_resident(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral, int *resident) {
+    if (!resident) return MG_ERR_INVALID;
+    *resident = resident_size(n, nnz, max_degree, integral);
+    return MG_OK;
+}
+
 mg_status mg_sweep_options(mg_ctx *ctx, const mg_sweep_opts *opts) {
     if (!ctx) return MG_ERR_INVALID;
     const int fill = opts ? opts->cluster_fill : MG_FILL_AUTO;

@@ -330,14 +330,19 @@ double modularity_from_acc(const SweepAcc &a, double mass, int integral);
 // flight than the class kernels, which counts once a sweep takes longer than
 // their launches.  SBM runs, local move only, resident / class kernels: 1.0 M
 // entries 2.5 / 5.5 ms, 4.0 M 5.2 / 8.1, 10 M 11.7 / 14.4, 24 M 29.0 / 25.7;
-// Chung-Lu, 15 M entries: 15.2 / 17.5 ms.
-constexpr uint64_t kResidentMaxEntries = 20u << 20;
+// Chung-Lu, 15 M entries: 15.2 / 17.5 ms.  Real weights, whose tables add doubles,
+// meet earlier.  Whole Chung-Lu runs, versions 2 and 1: 11.7 M entries 24.9 / 29.1
+// and 23.0 / 24.5 ms, 15.8 M 22.6 / 22.2 and 15.3 / 14.9, 17.6 M 42.3 / 40.9 and
+// 28.4 / 26.7 (integer weights of the same 17.6 M: 45.0 / 55.6 and 18.4 / 19.1).
+constexpr uint64_t kResidentMaxEntries = 20u << 20;      // integral weights
+constexpr uint64_t kResidentMaxEntriesReal = 14u << 20;  // real weights
 struct ResidentResult {
     int base = 0;                            // buffer holding the accepted assignment
     std::vector<double> Q;                   // per sweep: Q of its input assignment
     std::vector<unsigned long long> distinct;  // per sweep: candidate pairs
 };
-bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws);
+bool resident_size(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral);
+bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws, int integral);
 // Iterates the prepared level (k, sigma, C[0] set by level_init, classes by
 // move_prepare_level) to its end.
 void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,

@@ -153,7 +153,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         };
         // (the printed table has a time per iteration: verbose runs take the
         // iteration-by-iteration path)
-        if (!verbose && resident_level(cur, mlv, ctx->mws)) {
+        if (!verbose && resident_level(cur, mlv, ctx->mws, integral)) {
             resident = true;
             ResidentResult R;
             MG_CUDA(cudaEventRecord(ctx->ev[4], s));

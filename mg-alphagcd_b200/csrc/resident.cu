@@ -23,9 +23,14 @@ struct ResidentBlock {
 
 }  // namespace
 
-bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws) {
-    if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON || g.n == 0 || g.nnz > kResidentMaxEntries) return false;
-    return std::min(lvl.bins.max_degree, g.n) <= kResidentCapacity;
+bool resident_size(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral) {
+    if (n == 0 || nnz > (integral ? kResidentMaxEntries : kResidentMaxEntriesReal)) return false;
+    return std::min(max_degree, n) <= kResidentCapacity;
+}
+
+bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws, int integral) {
+    if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON) return false;
+    return resident_size(g.n, g.nnz, lvl.bins.max_degree, integral);
 }
 
 void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,

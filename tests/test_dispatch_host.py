@@ -44,3 +44,31 @@ def test_batch_team_bounds(mg):
     out = ct.c_int()
     assert mg.lib().mg_test_batch_team(1, None, 1, 148, ct.byref(out)) != 0
     assert mg.lib().mg_test_batch_team(0, None, 1, 0, ct.byref(out)) != 0
+
+
+def _resident(mg, n, nnz, max_degree, integral):
+    out = ct.c_int(-1)
+    assert mg.lib().mg_test_level_resident(n, nnz, max_degree, int(integral), ct.byref(out)) == 0
+    return out.value
+
+
+# ms of whole runs on a B200: resident kernels, class kernels (Chung-Lu graphs)
+@pytest.mark.parametrize("n,nnz,max_degree,integral,res,cls", [
+    (50000, 913494, 8000, False, 4.25, 7.09), (400000, 7806736, 8000, False, 11.07, 14.41),
+    (600000, 11672752, 12000, False, 24.88, 29.09), (600000, 11672752, 12000, False, 23.00, 24.48),
+    (800000, 15774034, 8000, False, 22.64, 22.24), (800000, 15774034, 8000, False, 15.32, 14.85),
+    (900000, 17630442, 12000, False, 42.33, 40.94), (900000, 17630442, 12000, False, 28.41, 26.68),
+    (1000000, 19764904, 8000, False, 31.00, 29.79),  # (class kernels: an earlier form of them)
+    (900000, 17630442, 12000, True, 44.97, 55.60), (900000, 17630442, 12000, True, 29.66, 35.93),
+])
+def test_level_resident(mg, n, nnz, max_degree, integral, res, cls):
+    assert _resident(mg, n, nnz, max_degree, integral) == (res < cls)
+
+
+def test_level_resident_bounds(mg):
+    for integral, most in ((True, 20 << 20), (False, 14 << 20)):
+        assert _resident(mg, 10**6, most, 500, integral) == 1
+        assert _resident(mg, 10**6, most + 1, 500, integral) == 0
+    assert _resident(mg, 0, 0, 0, True) == 0
+    assert _resident(mg, 10**6, 10**6, 14336, True) == 1 and _resident(mg, 10**6, 10**6, 14337, True) == 0
+    assert _resident(mg, 14336, 10**6, 10**6, True) == 1
