@@ -342,6 +342,11 @@ mg_status mg_test_batch_team(uint32_t graphs, const uint64_t *loads, int integra
 /* *resident = 1 when a run's level of n vertices, nnz entries and that largest
  * degree takes the resident kernel by default, 0 when the class kernels. */
 mg_status mg_test_level_resident(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral, int *resident);
+/* Limits of the resident kernels on a context: SMs that count as the device's (-1:
+ * its own; 0: none, the class kernels run), sweeps of one launch (0: built in) and
+ * polls of a grid barrier after which its blocks give up and the run goes on with
+ * the class kernels (0: built in).  Results do not depend on them. */
+mg_status mg_test_resident_limits(mg_ctx *ctx, int sms, int sweeps, uint32_t polls);
 
 /* ---- batched form --------------------------------------------------------------
  * No reference counterpart: the reference runs one graph per process.  A batch

@@ -123,7 +123,7 @@ EXPORTED = [
     "mg_tune_mode", "mg_tune_table", "mg_tune_save", "mg_tune_load", "mg_graph_generate_chunglu",
     "mg_graph_from_mtx_ex", "mg_csr_from_mtx", "mg_csr_info", "mg_csr_arrays", "mg_csr_free",
     "mg_result_level_map", "mg_result_level_csr", "mg_sweep_options", "mg_test_fail_allocation",
-    "mg_test_batch_team", "mg_test_level_resident",
+    "mg_test_batch_team", "mg_test_level_resident", "mg_test_resident_limits",
 ]
 TUNE_OFF, TUNE_CACHED, TUNE_ON = 0, 1, 2
 FILL_AUTO, FILL_OWN, FILL_SPLIT = 0, 1, 2
@@ -195,6 +195,7 @@ def lib():
     L.mg_test_fail_allocation.argtypes = [u64, ct.POINTER(u64)]
     L.mg_test_batch_team.argtypes = [u32, vp, i32, i32, ct.POINTER(i32)]
     L.mg_test_level_resident.argtypes = [u32, u64, u32, i32, ct.POINTER(i32)]
+    L.mg_test_resident_limits.argtypes = [vp, i32, i32, u32]
     L.mg_tune_table.argtypes = [vp, ct.c_char_p, ct.c_size_t, ct.POINTER(ct.c_size_t)]
     L.mg_tune_save.argtypes = [vp, ct.c_char_p]
     L.mg_tune_load.argtypes = [vp, ct.c_char_p]
@@ -322,6 +323,10 @@ class Context:
     def tune_mode(self, mode: int):
         """TUNE_OFF: built-in shapes; TUNE_CACHED: table only; TUNE_ON: also time new classes."""
         self.check(lib().mg_tune_mode(self.h, mode), "mg_tune_mode")
+
+    def resident_limits(self, sms: int = -1, sweeps: int = 0, polls: int = 0):
+        """Test hook (mg_test_resident_limits)."""
+        self.check(lib().mg_test_resident_limits(self.h, sms, sweeps, polls), "mg_test_resident_limits")
 
     def sweep_options(self, cluster_fill: int = FILL_AUTO, giant_class: int = 0,
                       coarsen_combine: int = COMBINE_AUTO, light_streams: int = 0,

@@ -502,23 +502,23 @@ int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vect
     std::vector<uint64_t> l;
     l.reserve(alive.size());
     for (uint32_t g : alive) l.push_back(load[g]);
-    return resident_team(l.data(), (uint32_t)l.size(), !integral, kNumSMs);
+    const int sms = ws.resident_sms();
+    return sms > 0 ? resident_team(l.data(), (uint32_t)l.size(), !integral, sms) : 0;
 }
 
-void launch_batch(const lmr::ResidentBatchArgs &A, int wk, const SweepParams &p, int ctas, unsigned most,
+bool launch_batch(const lmr::ResidentBatchArgs &A, int wk, const SweepParams &p, int ctas, unsigned most,
                   cudaStream_t s) {
-    if (wk == WK_UNIT) lmr::launch_batch_unit(A, p.precision, p.version, ctas, most, s);
-    else if (wk == WK_U32) lmr::launch_batch_u32(A, p.precision, p.version, ctas, most, s);
-    else if (wk == WK_F32I) lmr::launch_batch_f32i(A, p.precision, p.version, ctas, most, s);
-    else if (wk == WK_F64I) lmr::launch_batch_f64i(A, p.precision, p.version, ctas, most, s);
-    else if (wk == WK_F32) lmr::launch_batch_f32(A, p.precision, p.version, ctas, most, s);
-    else lmr::launch_batch_f64(A, p.precision, p.version, ctas, most, s);
+    const auto launch = wk == WK_UNIT ? lmr::launch_batch_unit : wk == WK_U32 ? lmr::launch_batch_u32
+                      : wk == WK_F32I ? lmr::launch_batch_f32i : wk == WK_F64I ? lmr::launch_batch_f64i
+                      : wk == WK_F32 ? lmr::launch_batch_f32 : lmr::launch_batch_f64;
+    return launch(A, p.precision, p.version, ctas, most, s);
 }
 
 // All iterations of the phase for the graphs `order` (largest first).  Leaves
 // what the iteration loop leaves: base buffers in the control words, Q and
-// iteration counts per graph.
-void resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLevel &lvl, const SweepParams &p,
+// iteration counts per graph.  False, with the phase's start as it was: the device
+// holds no such cluster.
+bool resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLevel &lvl, const SweepParams &p,
                     double thr, const uint32_t *goff, std::vector<uint32_t> order, int ctas, mg_summary &S,
                     cudaStream_t s) {
     using namespace lmr;
@@ -572,12 +572,16 @@ void resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLeve
     A.distinct = &ctx->mws.acc.get()->distinct;
     A.totals = &tail->totals;
     const int wk = p.integral ? (g.wk == WK_F32 ? (int)WK_F32I : g.wk == WK_F64 ? (int)WK_F64I : g.wk) : g.wk;
+    const MoveWorkspace &ws = ctx->mws;
+    A.sweeps = ws.test_sweeps > 0 ? std::min(ws.test_sweeps, kResidentBatchIters) : kResidentBatchIters;
+    const unsigned clusters = (unsigned)(ws.resident_sms() / ctas);
+    if (clusters == 0) return false;
     unsigned long long sweeps = 0;
     while (!order.empty()) {
         A.count = (uint32_t)order.size();
         MG_CUDA(cudaMemcpyAsync(d_order, order.data(), sizeof(uint32_t) * order.size(), cudaMemcpyHostToDevice, s));
         MG_CUDA(cudaMemsetAsync(tail, 0, sizeof(Tail), s));
-        launch_batch(A, wk, p, ctas, A.count, s);
+        if (!launch_batch(A, wk, p, ctas, std::min(A.count, clusters), s)) return false;
         Tail ht;
         MG_CUDA(cudaMemcpyAsync(&ht, tail, sizeof ht, cudaMemcpyDeviceToHost, s));
         MG_CUDA(cudaStreamSynchronize(s));
@@ -589,6 +593,7 @@ void resident_phase(mg_ctx *ctx, mg_batch *b, const GraphView &g, const MoveLeve
         order.erase(std::remove_if(order.begin(), order.end(), [&](uint32_t q) { return hs[q].done; }), order.end());
     }
     S.sweeps += sweeps;
+    return true;
 }
 
 }  // namespace
@@ -781,10 +786,12 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
             load[g] = hnnz[g] + 4ull * ng;
         }
         const int ctas = resident_ctas(ctx->mws, mlv, order, load, most_vertices, integral);
+        bool resident = false;
         if (ctas > 0) {
             std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return load[x] > load[y]; });
-            resident_phase(ctx, b, cur, mlv, sp, thr, goff, order, ctas, S, s);
-        } else {
+            resident = resident_phase(ctx, b, cur, mlv, sp, thr, goff, order, ctas, S, s);
+        }
+        if (!resident) {
             // active lists of the phase
             Lists Ls;
             rebuild_lists(ctx, W, mlv, Ls, true, n, s);

@@ -624,6 +624,14 @@ mg_status mg_test_level_resident(uint32_t n, uint64_t nnz, uint32_t max_degree, 
     return MG_OK;
 }
 
+mg_status mg_test_resident_limits(mg_ctx *ctx, int sms, int sweeps, uint32_t polls) {
+    if (!ctx || sms < -1 || sweeps < 0) return MG_ERR_INVALID;
+    ctx->mws.test_sms = sms;
+    ctx->mws.test_sweeps = sweeps;
+    ctx->mws.test_polls = polls;
+    return MG_OK;
+}
+
 mg_status mg_sweep_options(mg_ctx *ctx, const mg_sweep_opts *opts) {
     if (!ctx) return MG_ERR_INVALID;
     const int fill = opts ? opts->cluster_fill : MG_FILL_AUTO;

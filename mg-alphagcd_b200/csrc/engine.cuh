@@ -197,6 +197,12 @@ struct MoveWorkspace {
     // the resident kernels (blocks that take a whole SM) may run; not where
     // other contexts' work shares the device (a server with several slots)
     bool resident = true;
+    int sms = 0;  // SMs of the device (fewer than the part's on a partition of it)
+    // mg_test_resident_limits: SMs that count as the device's (-1: its own),
+    // sweeps of a launch and polls of a barrier (0: built in)
+    int test_sms = -1, test_sweeps = 0;
+    unsigned test_polls = 0;
+    int resident_sms() const { return test_sms < 0 || test_sms > sms ? sms : test_sms; }
     DBuf<unsigned char> res_block;  // resident level kernel: state, sums, counters, barrier
     void *h_resident = nullptr;    // pinned image of them
     DBuf<SmallInfo> small;         // counts of a small level
@@ -344,8 +350,10 @@ struct ResidentResult {
 bool resident_size(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral);
 bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws, int integral);
 // Iterates the prepared level (k, sigma, C[0] set by level_init, classes by
-// move_prepare_level) to its end.
-void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,
+// move_prepare_level) to its end.  False: the device holds no block of the kernel,
+// or its blocks did not meet at a barrier in time (other work kept some of them
+// from starting); the level's start is then to be prepared again.
+bool resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,
                   ResidentResult &out, cudaStream_t s);
 // CTAs per graph (1, 2, 4, 8) for a phase of a batch in the resident kernel, 0
 // when the class kernels serve it better (one graph among many that is too large

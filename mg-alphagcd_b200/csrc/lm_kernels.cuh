@@ -1477,6 +1477,22 @@ inline void raise_smem_limit(const void *kern, size_t smem) {
     done.insert({kern, dev});
 }
 
+// Blocks of a kernel that an SM holds, cached per device like the carveouts.
+inline int blocks_per_sm(const void *kern, unsigned block, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<const void *, unsigned, size_t, int>, int> cache;
+    int dev = 0;
+    MG_CUDA(cudaGetDevice(&dev));
+    const auto key = std::make_tuple(kern, block, smem, dev);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+    int blocks = 0;
+    MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, (int)block, smem));
+    cache.emplace(key, blocks);
+    return blocks;
+}
+
 // Shared-memory carveout (percent of the SM's 228 KB) that holds `blocks`
 // resident blocks of `smem` dynamic and `stat` static bytes each (plus the
 // per-block reserve); the rest of the SM's 256 KB stays L1, which the sweep

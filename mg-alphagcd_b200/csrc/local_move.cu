@@ -226,6 +226,9 @@ MoveWorkspace::~MoveWorkspace() {
 
 void MoveWorkspace::init_streams() {
     if (streams[0]) return;
+    int dev = 0;
+    MG_CUDA(cudaGetDevice(&dev));
+    MG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     for (auto &s : streams) MG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     MG_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     for (auto &e : ev_join) MG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -118,6 +118,7 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
     int phase = 0;
     MoveLevel mlv;
     bool prepared = false;  // the level's start came with its coarsening (small levels)
+    bool whole_sm = true;   // the resident kernel could run so far
     SweepParams sp;
     sp.version = version;
     sp.precision = o.precision;
@@ -153,12 +154,19 @@ void louvain_run(mg_ctx *ctx, const mg_graph *g, const mg_run_opts &o, mg_result
         };
         // (the printed table has a time per iteration: verbose runs take the
         // iteration-by-iteration path)
-        if (!verbose && resident_level(cur, mlv, ctx->mws, integral)) {
-            resident = true;
-            ResidentResult R;
+        ResidentResult R;
+        if (!verbose && whole_sm && resident_level(cur, mlv, ctx->mws, integral)) {
             MG_CUDA(cudaEventRecord(ctx->ev[4], s));
-            resident_run(ctx, cur, mlv, sp, thr, R, s);
+            resident = resident_run(ctx, cur, mlv, sp, thr, R, s);
             MG_CUDA(cudaEventRecord(ctx->ev[5], s));
+            if (!resident) {  // the class kernels serve the rest of the run
+                whole_sm = false;
+                level_init(cur, k, sigma, C[0], s, false);
+                move_prepare_level(cur, mlv, ctx->mws, s);
+                level_init_long(cur, mlv, k, sigma, s);
+            }
+        }
+        if (resident) {
             phase_lm += tp.stop_sync();
             float ms = 0;
             MG_CUDA(cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]));

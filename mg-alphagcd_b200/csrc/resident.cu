@@ -33,7 +33,7 @@ bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspac
     return resident_size(g.n, g.nnz, lvl.bins.max_degree, integral);
 }
 
-void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,
+bool resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,
                   ResidentResult &out, cudaStream_t s) {
     MoveWorkspace &ws = ctx->mws;
     const Bins &B = lvl.bins;
@@ -60,11 +60,14 @@ void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const S
     A.bits = resident_bits(std::min(B.max_degree, g.n));
     for (int c = 0; c < kSweepClasses; c++) A.cls[c] = B.offset[c];
     A.cls[kSweepClasses] = g.n;
-    // CTAs: work for half of a CTA's warps, or as many as there are SMs
+    A.sweeps = ws.test_sweeps > 0 ? std::min(ws.test_sweeps, kResidentIters) : kResidentIters;
+    A.polls = ws.test_polls ? ws.test_polls : kBarrierPolls;
+    A.sms = ws.resident_sms();
+    // CTAs: work for half of a CTA's warps, or as many as the device holds
     uint64_t warps = 0;
     for (int c = 0; c < kSweepClasses; c++)
         warps += c > 5 ? B.size[c] * ceil_div(1ull << c, 1ull << (A.bits - 6)) : ceil_div(B.size[c], kTileU * (32u >> c));
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(warps, 16), kNumSMs));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(warps, 16), 0xffffu));
     A.state = &db->state;
     A.acc = db->acc;
     A.task_ctr = db->task_ctr;
@@ -84,22 +87,21 @@ void resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const S
         hb->state = st;
         hb->state.iters = 0;
         MG_CUDA(cudaMemcpyAsync(db, hb, sizeof *hb, cudaMemcpyHostToDevice, s));
-        if (wk == WK_UNIT) launch_resident_unit(A, p.precision, p.version, grid, s);
-        else if (wk == WK_U32) launch_resident_u32(A, p.precision, p.version, grid, s);
-        else if (wk == WK_F32I) launch_resident_f32i(A, p.precision, p.version, grid, s);
-        else if (wk == WK_F64I) launch_resident_f64i(A, p.precision, p.version, grid, s);
-        else if (wk == WK_F32) launch_resident_f32(A, p.precision, p.version, grid, s);
-        else launch_resident_f64(A, p.precision, p.version, grid, s);
+        const auto launch = wk == WK_UNIT ? launch_resident_unit : wk == WK_U32 ? launch_resident_u32
+                          : wk == WK_F32I ? launch_resident_f32i : wk == WK_F64I ? launch_resident_f64i
+                          : wk == WK_F32 ? launch_resident_f32 : launch_resident_f64;
+        if (!launch(A, p.precision, p.version, grid, s)) return false;
         MG_CUDA(cudaMemcpyAsync(hb, db, sizeof(ResidentState) + sizeof(SweepAcc) * kResidentIters,
                                 cudaMemcpyDeviceToHost, s));
         MG_CUDA(cudaStreamSynchronize(s));
-        MG_CHECK(!hb->state.err, MG_ERR_TIMEOUT, "resident level: a grid barrier was not reached by every block");
+        if (hb->state.err) return false;
         for (int i = 0; i < hb->state.iters; i++) {
             out.Q.push_back(hb->acc[i].pad);
             out.distinct.push_back(hb->acc[i].distinct);
         }
     } while (!hb->state.done);
     out.base = hb->state.base;
+    return true;
 }
 
 }  // namespace mg

@@ -368,11 +368,12 @@ __device__ __forceinline__ void hash_vertex(const AV &A, const uint32_t *P, uint
 
 // Grid barrier (cooperative launch: all CTAs are resident).  The counter only
 // grows; `target` is the count that completes this barrier.  Thread 0 gives up
-// after kBarrierSpins polls (seconds), which ends the kernel with an error.
-__device__ __forceinline__ bool grid_wait(unsigned *ctr, unsigned target) {
+// after `polls` polls (seconds), which ends the kernel with an error: blocks of
+// the launch may not have started, held back by other work on the device.
+__device__ __forceinline__ bool grid_wait(unsigned *ctr, unsigned target, unsigned polls) {
     __threadfence();
     atomicAdd(ctr, 1u);
-    for (unsigned spin = 0; spin < kBarrierSpins; spin++) {
+    for (unsigned spin = 0; spin < polls; spin++) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
         if (v >= target) {
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A
     __syncthreads();
     unsigned bar = 0;  // barriers passed (thread 0)
     const uint32_t gthreads = gridDim.x * kThreads, gt = blockIdx.x * kThreads + t;
-    for (int it = 0; it < kResidentIters; it++) {
+    for (int it = 0; it < A.sweeps; it++) {
         SweepAcc *acc = A.acc + it;
         const uint32_t *P = A.C[sh.st.p];
         uint32_t *N = A.C[sh.st.nx];
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A
             }
             if (r.distinct) atomicAdd(&acc->distinct, r.distinct);
             bar++;
-            sh.ok = grid_wait(A.barrier, bar * gridDim.x);
+            sh.ok = grid_wait(A.barrier, bar * gridDim.x, A.polls);
             const double x = A.integral ? __ull2double_rn(__ldcg(&acc->sin_u)) : __ldcg(&acc->sin_f);
             const double y = A.integral ? __ull2double_rn(__ldcg(&acc->s2_u)) : __ldcg(&acc->s2_f);
             const double Q = sweep_q(x, y, A.mass);
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_kernel(ResidentArgs A
         __syncthreads();
         if (t == 0) {
             bar++;
-            sh.ok = grid_wait(A.barrier, bar * gridDim.x);
+            sh.ok = grid_wait(A.barrier, bar * gridDim.x, A.polls);
         }
         __syncthreads();
         if (!sh.ok) {
@@ -688,7 +689,7 @@ __global__ void __launch_bounds__(kThreads, 1) lm_resident_batch_kernel(Resident
         if (t == 0) count_tasks(sh, A.bits, size);
         __syncthreads();
         // (iterations of a launch are bounded; the host launches again)
-        for (int it = 0; it < kResidentBatchIters && !sh.st.done; it++) {
+        for (int it = 0; it < A.sweeps && !sh.st.done; it++) {
             const int par = it & 1;
             const uint32_t *P = A.C[sh.st.p];
             uint32_t *N = A.C[sh.st.nx];
@@ -744,12 +745,15 @@ size_t resident_smem(int bits) {
     return ((size_t)1 << bits) * (sizeof(typename ValT<WK>::type) + sizeof(uint32_t) + 1);
 }
 
+// At most `grid` CTAs, and as many as run at once.
 template <int WK, int PREC, int VER>
-void launch_resident(const ResidentArgs &A, unsigned grid, cudaStream_t s) {
+bool launch_resident(const ResidentArgs &A, unsigned grid, cudaStream_t s) {
     auto kern = lm_resident_kernel<WK, PREC, VER>;
     raise_smem_limit((const void *)kern, resident_smem<WK>(kResidentMaxBits));
+    const unsigned fit = (unsigned)(blocks_per_sm((const void *)kern, kThreads, resident_smem<WK>(A.bits)) * A.sms);
+    if (fit == 0) return false;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(std::min(grid, fit));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = resident_smem<WK>(A.bits);
     cfg.stream = s;
@@ -758,8 +762,14 @@ void launch_resident(const ResidentArgs &A, unsigned grid, cudaStream_t s) {
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    MG_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, A);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports
+        cudaGetLastError();
+        return false;
+    }
+    MG_CUDA(e);
     MG_LAUNCH_CHECK();
+    return true;
 }
 
 template <int WK, int PREC, int VER>
@@ -782,62 +792,45 @@ cudaLaunchConfig_t batch_config(const ResidentBatchArgs &A, int ctas, unsigned g
 
 // As many clusters of `ctas` CTAs as the device holds, at most `most`.
 template <int WK, int PREC, int VER>
-void launch_batch(const ResidentBatchArgs &A, int ctas, unsigned most, cudaStream_t s) {
+bool launch_batch(const ResidentBatchArgs &A, int ctas, unsigned most, cudaStream_t s) {
     auto kern = lm_resident_batch_kernel<WK, PREC, VER>;
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = batch_config<WK, PREC, VER>(A, ctas, (unsigned)ctas, s, at);
     int fit = 0;
     MG_CUDA(cudaOccupancyMaxActiveClusters(&fit, (void *)kern, &cfg));
-    MG_CHECK(fit > 0, MG_ERR_UNSUPPORTED, "cluster shape cannot be scheduled on this device");
+    if (fit == 0) return false;
     cfg.gridDim = dim3(std::min((unsigned)fit, most) * (unsigned)ctas);
     MG_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
     MG_LAUNCH_CHECK();
+    return true;
 }
 
 template <int WK>
-void launch_batch_kind(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
+bool launch_batch_kind(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
     auto version = [&](auto precc) {
         constexpr int PREC = decltype(precc)::value;
-        if (ver == 1) launch_batch<WK, PREC, 1>(A, ctas, most, s);
-        else launch_batch<WK, PREC, 2>(A, ctas, most, s);
+        return ver == 1 ? launch_batch<WK, PREC, 1>(A, ctas, most, s)
+                        : launch_batch<WK, PREC, 2>(A, ctas, most, s);
     };
-    if (prec == MG_PREC_FP64) {
-        version(std::integral_constant<int, MG_PREC_FP64>());
-        return;
-    }
-    if (prec == MG_PREC_FP32) {
-        version(std::integral_constant<int, MG_PREC_FP32>());
-        return;
-    }
+    if (prec == MG_PREC_FP64) return version(std::integral_constant<int, MG_PREC_FP64>());
+    if (prec == MG_PREC_FP32) return version(std::integral_constant<int, MG_PREC_FP32>());
     if constexpr (kIntg<WK>) {
-        if (prec == MG_PREC_INT64) {
-            version(std::integral_constant<int, MG_PREC_INT64>());
-            return;
-        }
+        if (prec == MG_PREC_INT64) return version(std::integral_constant<int, MG_PREC_INT64>());
     }
     throw Error(MG_ERR_INVALID, "unknown weight kind or precision");
 }
 
 template <int WK>
-void launch_resident_kind(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
+bool launch_resident_kind(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
     auto version = [&](auto precc) {
         constexpr int PREC = decltype(precc)::value;
-        if (ver == 1) launch_resident<WK, PREC, 1>(A, grid, s);
-        else launch_resident<WK, PREC, 2>(A, grid, s);
+        return ver == 1 ? launch_resident<WK, PREC, 1>(A, grid, s)
+                        : launch_resident<WK, PREC, 2>(A, grid, s);
     };
-    if (prec == MG_PREC_FP64) {
-        version(std::integral_constant<int, MG_PREC_FP64>());
-        return;
-    }
-    if (prec == MG_PREC_FP32) {
-        version(std::integral_constant<int, MG_PREC_FP32>());
-        return;
-    }
+    if (prec == MG_PREC_FP64) return version(std::integral_constant<int, MG_PREC_FP64>());
+    if (prec == MG_PREC_FP32) return version(std::integral_constant<int, MG_PREC_FP32>());
     if constexpr (kIntg<WK>) {
-        if (prec == MG_PREC_INT64) {
-            version(std::integral_constant<int, MG_PREC_INT64>());
-            return;
-        }
+        if (prec == MG_PREC_INT64) return version(std::integral_constant<int, MG_PREC_INT64>());
     }
     throw Error(MG_ERR_INVALID, "unknown weight kind or precision");
 }

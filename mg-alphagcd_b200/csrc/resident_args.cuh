@@ -10,7 +10,7 @@ namespace lmr {
 constexpr int kResidentThreads = 1024;
 constexpr int kResidentIters = 48;     // iterations of one launch (the host launches again while a level goes on)
 constexpr int kResidentMaxBits = 14;   // slots of a CTA's table: 2^14 (9 or 13 bytes each)
-constexpr unsigned kBarrierSpins = 1u << 24;
+constexpr unsigned kBarrierPolls = 1u << 24;
 // warp steps of a tile task in flight at once: SBM runs of 4.0 M entries took
 // 5.8 ms of kernel time with 1, 5.0 ms with 2, 5.6 ms with 3 and 5.3 ms with 4
 // (spills)
@@ -48,6 +48,9 @@ struct ResidentArgs {
     unsigned long long nnz;
     int integral;
     int bits;  // log2 of the CTA's table slots
+    int sweeps;      // iterations of this launch, at most kResidentIters
+    unsigned polls;  // of a barrier before a block gives up
+    int sms;         // (launcher) SMs of the device
     uint32_t cls[kSweepClasses + 1];  // start of every degree class in the class list; n
     ResidentState *state;
     SweepAcc *acc;       // one per iteration, zeroed; pad receives Q
@@ -72,6 +75,7 @@ struct ResidentBatchArgs {
     uint32_t *C[3];
     double thr;
     int integral, bits;
+    int sweeps;             // iterations of a graph in this launch
     const uint32_t *cls;    // per graph: start of its part of every degree class (graphs + 1 rows)
     const uint32_t *goff;   // first vertex of each graph
     const uint32_t *gnnz;
@@ -88,17 +92,19 @@ struct ResidentBatchArgs {
 };
 
 #define MG_RESIDENT_KINDS(X) X(unit) X(u32) X(f32i) X(f64i) X(f32) X(f64)
+// The launchers return false, with nothing launched, when the device holds no
+// block (no cluster) of the kernel.
 #define MG_RESIDENT_BATCH(k) \
-    void launch_batch_##k(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s);
+    bool launch_batch_##k(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s);
 MG_RESIDENT_KINDS(MG_RESIDENT_BATCH)
 #undef MG_RESIDENT_BATCH
 
-void launch_resident_unit(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
-void launch_resident_u32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
-void launch_resident_f32i(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
-void launch_resident_f64i(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
-void launch_resident_f32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
-void launch_resident_f64(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
+bool launch_resident_unit(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
+bool launch_resident_u32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
+bool launch_resident_f32i(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
+bool launch_resident_f64i(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
+bool launch_resident_f32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
+bool launch_resident_f64(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s);
 
 }  // namespace lmr
 }  // namespace mg

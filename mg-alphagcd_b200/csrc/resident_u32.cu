@@ -4,12 +4,12 @@
 namespace mg {
 namespace lmr {
 
-void launch_resident_u32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
-    launch_resident_kind<WK_U32>(A, prec, ver, grid, s);
+bool launch_resident_u32(const ResidentArgs &A, int prec, int ver, unsigned grid, cudaStream_t s) {
+    return launch_resident_kind<WK_U32>(A, prec, ver, grid, s);
 }
 
-void launch_batch_u32(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
-    launch_batch_kind<WK_U32>(A, prec, ver, ctas, most, s);
+bool launch_batch_u32(const ResidentBatchArgs &A, int prec, int ver, int ctas, unsigned most, cudaStream_t s) {
+    return launch_batch_kind<WK_U32>(A, prec, ver, ctas, most, s);
 }
 
 }  // namespace lmr
