@@ -62,6 +62,12 @@ const char *mg_version(void);
  * no MPI / NVSHMEM init is needed on one GPU. */
 mg_status mg_init(mg_ctx **ctx, const mg_opts *opts /* may be NULL */);
 mg_status mg_destroy(mg_ctx *ctx);
+/* A context keeps up to 256 MB of device buffers of graphs that were destroyed
+ * (given back by itself when any context of the process runs out of memory) and
+ * up to 256 MB of page-locked host memory that results are copied through.  mg_trim
+ * frees both now, for other users of the device; later calls make them anew.  The
+ * byte counts (either may be NULL) receive what was freed. */
+mg_status mg_trim(mg_ctx *ctx, size_t *device_bytes, size_t *host_bytes);
 const char *mg_last_error(const mg_ctx *ctx);
 
 /* ---- graphs -------------------------------------------------------------- */

@@ -123,7 +123,7 @@ EXPORTED = [
     "mg_tune_mode", "mg_tune_table", "mg_tune_save", "mg_tune_load", "mg_graph_generate_chunglu",
     "mg_graph_from_mtx_ex", "mg_csr_from_mtx", "mg_csr_info", "mg_csr_arrays", "mg_csr_free",
     "mg_result_level_map", "mg_result_level_csr", "mg_sweep_options", "mg_test_fail_allocation",
-    "mg_test_batch_team", "mg_test_level_resident", "mg_test_resident_limits",
+    "mg_test_batch_team", "mg_test_level_resident", "mg_test_resident_limits", "mg_trim",
 ]
 TUNE_OFF, TUNE_CACHED, TUNE_ON = 0, 1, 2
 FILL_AUTO, FILL_OWN, FILL_SPLIT = 0, 1, 2
@@ -195,6 +195,7 @@ def lib():
     L.mg_test_fail_allocation.argtypes = [u64, ct.POINTER(u64)]
     L.mg_test_batch_team.argtypes = [u32, vp, i32, i32, ct.POINTER(i32)]
     L.mg_test_level_resident.argtypes = [u32, u64, u32, i32, ct.POINTER(i32)]
+    L.mg_trim.argtypes = [vp, ct.POINTER(ct.c_size_t), ct.POINTER(ct.c_size_t)]
     L.mg_test_resident_limits.argtypes = [vp, i32, i32, u32]
     L.mg_tune_table.argtypes = [vp, ct.c_char_p, ct.c_size_t, ct.POINTER(ct.c_size_t)]
     L.mg_tune_save.argtypes = [vp, ct.c_char_p]
@@ -241,6 +242,13 @@ class Context:
                 child.close()
             lib().mg_destroy(self.h)
             self.h = ct.c_void_p()
+
+    def trim(self) -> tuple:
+        """Free the device buffers and the page-locked memory that the context
+        keeps for later calls (mg_trim); returns their bytes."""
+        d, h = ct.c_size_t(), ct.c_size_t()
+        self.check(lib().mg_trim(self.h, ct.byref(d), ct.byref(h)), "mg_trim")
+        return d.value, h.value
 
     def _adopt(self, child):
         if not hasattr(self, "_children"):

@@ -24,10 +24,6 @@ mg_status fail(mg_ctx *ctx, mg_status st, const std::string &msg) {
 
 template <class F>
 mg_status guarded(mg_ctx *ctx, F &&f) {
-    struct Pool {  // allocations of this entry point may draw on the context's pool
-        explicit Pool(BufPool *p) { t_pool = p; }
-        ~Pool() { t_pool = nullptr; }
-    } pool(ctx ? &ctx->pool : nullptr);
     try {
         if (ctx) MG_CUDA(cudaSetDevice(ctx->device));
         f();
@@ -63,7 +59,6 @@ mg_ctx::~mg_ctx() {
 
 namespace mg {
 thread_local unsigned long long g_kernel_launches = 0;
-thread_local BufPool *t_pool = nullptr;
 
 static std::atomic<long long> g_alloc_fault_countdown{0};  // 0: disarmed
 
@@ -137,6 +132,18 @@ mg_status mg_destroy(mg_ctx *ctx) {
     cudaSetDevice(ctx->device);
     delete ctx;
     return MG_OK;
+}
+
+mg_status mg_trim(mg_ctx *ctx, size_t *device_bytes, size_t *host_bytes) {
+    if (!ctx) return MG_ERR_INVALID;
+    size_t d = 0, h = 0;
+    const mg_status st = guarded(ctx, [&] {
+        d = ctx->pool.trim();
+        if (ctx->spare) h = ctx->spare->trim();
+    });
+    if (device_bytes) *device_bytes = d;
+    if (host_bytes) *host_bytes = h;
+    return st;
 }
 
 const char *mg_last_error(const mg_ctx *ctx) { return ctx ? ctx->last_error.c_str() : g_orphan_error.c_str(); }

@@ -74,17 +74,31 @@ bool alloc_fault_due();
 // Device buffers of graphs that ended, kept by their context for the next ones:
 // a graph that is uploaded, used once and dropped otherwise pays a cudaMalloc
 // and a cudaFree (which waits for the device) per array.  At most kBytes and
-// kCount buffers are kept; they go back when the context ends or an allocation
-// finds no memory.  All work on a context's buffers is ordered by its stream,
-// so a buffer may be handed out while kernels of its last user still run.
+// kCount buffers are kept, the newest ones (the oldest go first, so that sizes
+// that no longer come do not hold the places); they go back when the context
+// ends, when mg_trim asks for it, or when an allocation of any context of the
+// process finds no memory.  All work on a context's buffers is ordered by its
+// stream, so a buffer may be handed out while kernels of its last user still run.
 class BufPool {
 public:
     static constexpr size_t kBytes = 256u << 20;
     static constexpr size_t kCount = 32;
-    BufPool() = default;
+    BufPool() {
+        kept_.reserve(kCount + 1);
+        std::lock_guard<std::mutex> lk(all().mu);
+        all().pools.push_back(this);
+    }
     BufPool(const BufPool &) = delete;
     BufPool &operator=(const BufPool &) = delete;
-    ~BufPool() { trim(); }
+    ~BufPool() {
+        {
+            std::lock_guard<std::mutex> lk(all().mu);
+            auto &p = all().pools;
+            for (size_t i = 0; i < p.size(); i++)
+                if (p[i] == this) p.erase(p.begin() + (long)i--);
+        }
+        trim();
+    }
     // the smallest kept buffer of at least `bytes` and not far above; null: none
     void *take(size_t bytes, size_t &got) {
         std::lock_guard<std::mutex> lk(mu_);
@@ -94,38 +108,57 @@ public:
                 (best == kept_.size() || kept_[i].second < kept_[best].second))
                 best = i;
         if (best == kept_.size()) return nullptr;
-        void *p = kept_[best].first;
         got = kept_[best].second;
-        total_ -= got;
-        kept_.erase(kept_.begin() + (long)best);
-        return p;
+        return remove(best);
     }
     void give(void *p, size_t bytes) {
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            if (total_ + bytes <= kBytes && kept_.size() < kCount) {
-                kept_.emplace_back(p, bytes);
-                total_ += bytes;
-                return;
-            }
+        if (bytes > kBytes) {
+            cudaFree(p);
+            return;
         }
-        cudaFree(p);
+        std::unique_lock<std::mutex> lk(mu_);
+        kept_.emplace_back(p, bytes);
+        total_ += bytes;
+        while (total_ > kBytes || kept_.size() > kCount) {
+            void *old = remove(0);
+            lk.unlock();
+            cudaFree(old);
+            lk.lock();
+        }
     }
-    void trim() {
+    // frees what is kept; returns its bytes
+    size_t trim() {
         std::lock_guard<std::mutex> lk(mu_);
+        const size_t bytes = total_;
         for (auto &b : kept_) cudaFree(b.first);
         kept_.clear();
         total_ = 0;
+        return bytes;
+    }
+    static void trim_all() {
+        std::lock_guard<std::mutex> lk(all().mu);
+        for (BufPool *p : all().pools) p->trim();
     }
 
 private:
+    struct Registry {
+        std::mutex mu;
+        std::vector<BufPool *> pools;
+    };
+    static Registry &all() {
+        static Registry *r = new Registry;  // (contexts may end after static objects)
+        return *r;
+    }
+    void *remove(size_t i) {
+        void *p = kept_[i].first;
+        total_ -= kept_[i].second;
+        kept_.erase(kept_.begin() + (long)i);
+        return p;
+    }
     std::mutex mu_;
-    std::vector<std::pair<void *, size_t>> kept_;
+    std::vector<std::pair<void *, size_t>> kept_;  // oldest first
     size_t total_ = 0;
 };
-
-// The pool of the context whose entry point this thread is in (null: none).
-extern thread_local BufPool *t_pool;
 
 // Grow-only device allocation owned by the engine (cudaMalloc on growth only),
 // from and back to a pool where it has one.
@@ -163,10 +196,10 @@ struct DBuf {
                 cap = roomy;
                 return p;
             }
-            // once more as asked, with what the context's pool holds given back
+            // once more as asked, with what the contexts' pools hold given back
             cudaGetLastError();
             p = nullptr;
-            if (t_pool) t_pool->trim();
+            BufPool::trim_all();
             MG_CUDA(cudaMalloc(&p, want * sizeof(T)));
             cap = want;
         }

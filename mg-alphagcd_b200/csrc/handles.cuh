@@ -25,9 +25,17 @@ struct PinnedSpare {
     std::mutex mu;
     uint32_t *p = nullptr;
     size_t cap = 0;
-    ~PinnedSpare() {
-        if (p) cudaFreeHost(p);
+    // frees the buffer (unless a result holds it); returns its bytes
+    size_t trim() {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!p) return 0;
+        const size_t bytes = cap * sizeof(uint32_t);
+        cudaFreeHost(p);
+        p = nullptr;
+        cap = 0;
+        return bytes;
     }
+    ~PinnedSpare() { trim(); }
 };
 class HostIds {
 public:
