@@ -24,17 +24,24 @@ mg_status fail(mg_ctx *ctx, mg_status st, const std::string &msg) {
 
 template <class F>
 mg_status guarded(mg_ctx *ctx, F &&f) {
+    mg_status st = MG_OK;
+    std::string msg;
     try {
         if (ctx) MG_CUDA(cudaSetDevice(ctx->device));
         f();
         return MG_OK;
     } catch (const Error &e) {
-        return fail(ctx, e.status, e.what());
+        st = e.status;
+        msg = e.what();
     } catch (const std::bad_alloc &) {
-        return fail(ctx, MG_ERR_OOM, "host allocation failed");
+        st = MG_ERR_OOM;
+        msg = "host allocation failed";
     } catch (const std::exception &e) {
-        return fail(ctx, MG_ERR_INVALID, e.what());
+        st = MG_ERR_INVALID;
+        msg = e.what();
     }
+    if (ctx) ctx_quiesce(ctx);
+    return fail(ctx, st, msg);
 }
 
 // copy a host assignment to the device and check every id is < n
@@ -72,6 +79,13 @@ bool alloc_fault_due() {
 
 // error text for entry points that run without a context (mg_last_error(NULL))
 void set_orphan_error(const std::string &msg) { g_orphan_error = msg; }
+
+void ctx_quiesce(mg_ctx *ctx) {
+    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    for (cudaStream_t s : ctx->mws.streams)
+        if (s) cudaStreamSynchronize(s);
+    cudaGetLastError();
+}
 
 void ctx_prepare(mg_ctx *ctx) {
     if (ctx->stream) return;

@@ -251,6 +251,10 @@ struct mg_batch_result {
 namespace mg {
 
 void ctx_prepare(mg_ctx *ctx);
+// After a call that failed: waits for what it had queued (copies from the caller's
+// page-locked arrays, kernels on buffers that are back in the pool) and forgets the
+// error, which the call reports, so that no later launch check finds it.
+void ctx_quiesce(mg_ctx *ctx);
 // error text for entry points that run without a context (mg_last_error(NULL))
 void set_orphan_error(const std::string &msg);
 // graph construction

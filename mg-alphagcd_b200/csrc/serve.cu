@@ -178,6 +178,7 @@ void run_batch(mg_server *S, mg_ctx *ctx, mg_batch *b, const std::vector<Job *> 
         msg = e.what();
     }
     if (st != MG_OK) {
+        ctx_quiesce(ctx);
         std::lock_guard<std::mutex> lk(S->mu);
         S->last_error = msg;
         for (Job *j : take)

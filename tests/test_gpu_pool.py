@@ -74,3 +74,32 @@ def test_another_contexts_allocation_gets_the_memory(mg):
         torch.cuda.empty_cache()
     a.close()
     b.close()
+
+
+def test_a_failed_call_leaves_no_copy_in_flight(mg):
+    """The third allocation of an upload fails while the offsets (240 MB of
+    page-locked memory, 4 ms on the link) are being copied: they are the
+    caller's again when the call returns, so the device is idle then."""
+    import time
+
+    import torch
+
+    n = 30_000_000
+    off = torch.zeros(n + 1, dtype=torch.int64).pin_memory().numpy().view(np.uint64)
+    c = mg.Context(0)
+    c.graph_from_csr(n, off, np.zeros(0, np.uint32)).close()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        c.trim()
+        mg.fail_allocation(3)
+        try:
+            with pytest.raises(mg.MGError) as e:
+                c.graph_from_csr(n, off, np.zeros(0, np.uint32))
+            t0 = time.perf_counter()
+            torch.cuda.synchronize()
+            waited = time.perf_counter() - t0
+        finally:
+            assert mg.fail_allocation(0) == 0
+        assert e.value.status == 3 and waited < 1e-3, waited
+    assert c.graph_from_csr(9, *_ring(9)).info()["nnz"] == 36
+    c.close()
