@@ -497,7 +497,7 @@ __global__ void class_starts_kernel(const uint32_t *perm, Idx19 off, const uint3
 
 int resident_ctas(const MoveWorkspace &ws, const MoveLevel &lvl, const std::vector<uint32_t> &alive,
                   const std::vector<uint64_t> &load, uint32_t most_vertices, int integral) {
-    if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON || alive.empty()) return 0;
+    if (!resident_allowed(ws) || alive.empty()) return 0;
     if (std::min(lvl.bins.max_degree, most_vertices) > lmr::kResidentCapacity) return 0;
     std::vector<uint64_t> l;
     l.reserve(alive.size());
@@ -770,15 +770,15 @@ void batch_run(mg_batch *b, const mg_run_opts &o, int flags, mg_batch_result &re
                                                                      W.loops.get(), ctrl);
         MG_LAUNCH_CHECK();
         level_init(cur, k, sigma, C[0], s, false);
-        if (phase > 0)  // (level 0: the batch's own entry offsets)
+        const bool choose = resident_allowed(ctx->mws);
+        if (phase > 0 && choose)  // (level 0: the batch's own entry offsets)
             MG_CUDA(cudaMemcpyAsync(hnnz.data(), W.gnnz.get(), sizeof(uint32_t) * G, cudaMemcpyDeviceToHost, s));
-        move_prepare_level(cur, mlv, ctx->mws, s);
+        move_prepare_level(cur, mlv, ctx->mws, s);  // (waits for the stream)
         level_init_long(cur, mlv, k, sigma, s);
-        MG_CUDA(cudaStreamSynchronize(s));
         sweep_reset_acc(ctx->mws, s);
         std::vector<uint32_t> order;
         uint32_t most_vertices = 0;
-        for (uint32_t g = 0; g < G; g++) {
+        for (uint32_t g = 0; g < G && choose; g++) {
             if (!alive[g]) continue;
             order.push_back(g);
             const uint32_t ng = hgoff[g + 1] - hgoff[g];

@@ -347,6 +347,9 @@ struct ResidentResult {
     std::vector<double> Q;                   // per sweep: Q of its input assignment
     std::vector<unsigned long long> distinct;  // per sweep: candidate pairs
 };
+inline bool resident_allowed(const MoveWorkspace &ws) {
+    return ws.resident && !ws.forced_policy && ws.tune.mode == MG_TUNE_ON;
+}
 bool resident_size(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral);
 bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws, int integral);
 // Iterates the prepared level (k, sigma, C[0] set by level_init, classes by

@@ -29,8 +29,7 @@ bool resident_size(uint32_t n, uint64_t nnz, uint32_t max_degree, int integral) 
 }
 
 bool resident_level(const GraphView &g, const MoveLevel &lvl, const MoveWorkspace &ws, int integral) {
-    if (!ws.resident || ws.forced_policy || ws.tune.mode != MG_TUNE_ON) return false;
-    return resident_size(g.n, g.nnz, lvl.bins.max_degree, integral);
+    return resident_allowed(ws) && resident_size(g.n, g.nnz, lvl.bins.max_degree, integral);
 }
 
 bool resident_run(mg_ctx *ctx, const GraphView &g, const MoveLevel &lvl, const SweepParams &p, double thr,
