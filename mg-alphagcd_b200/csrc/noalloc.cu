@@ -83,7 +83,7 @@ __device__ __forceinline__ double nb_double(double x) { return x; }
 
 // log2 of the slots of a vertex of degree d: at least 2 * d and 16, at most 2^most
 __device__ __forceinline__ int nb_bits(uint32_t d, int most) {
-    const int want = d <= 8 ? 4 : 33 - __clz(2 * d - 1);
+    const int want = d <= 8 ? 4 : 32 - __clz(2 * d - 1);
     return want < most ? want : most;
 }
 
