@@ -189,6 +189,23 @@ __global__ void __launch_bounds__(kExpandThreads) inner_weight_kernel(const uint
     flush_acc(acc, integral, sin, 0);
 }
 
+// The same where rows are mostly empty: a tile's block would walk kSparseRows rows
+// and more to find those of its 4,096 edges, so every edge searches its own (16.8 M
+// vertices, 4,000 entries, call with a 10 ms upload: 22.6 ms by tiles).
+constexpr uint32_t kSparseRows = 65536;
+template <int WK>
+__global__ void __launch_bounds__(256) inner_weight_sparse_kernel(const uint32_t *off, const uint32_t *col,
+                                                                  const void *w, uint32_t n, uint64_t m,
+                                                                  const uint32_t *C, int integral, SweepAcc *acc) {
+    double sin = 0;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
+        const bool in = C[col[e]] == C[last_row_at(off, n, e)];
+        if constexpr (WK == WK_UNIT) sin += in ? 1.0 : 0.0;
+        else sin += in ? wload<WK>(w, (uint32_t)e) : 0.0;
+    }
+    flush_acc(acc, integral, sin, 0);
+}
+
 // Largest cluster size (8 or 16) the device schedules for the heavy tiers.
 // (the largest tier: 16 CTAs for real weights, 8 dense CTAs for integral ones)
 int probe_max_cluster() {
@@ -406,15 +423,19 @@ void modularity_terms(const GraphView &g, const uint32_t *C, int integral, doubl
     sigma_sumsq(sigma, g.n, integral, ws, s);
     if (g.nnz == 0) return;
     SweepAcc *acc = ws.acc.ensure(1);
-    const unsigned grid = (unsigned)std::min<uint64_t>(ceil_div(g.nnz, kExpandTile), 148ull * 8);
-    auto run = [&](auto kern) {
-        kern<<<grid, kExpandThreads, 0, s>>>(g.off, g.col, g.w, g.n, g.nnz, C, integral, acc);
+    const uint64_t tiles = ceil_div(g.nnz, kExpandTile);
+    const bool sparse = g.n / tiles >= kSparseRows;
+    const unsigned grid = (unsigned)std::min<uint64_t>(sparse ? ceil_div(g.nnz, 256) : tiles, 148ull * 8);
+    static_assert(kExpandThreads == 256, "both forms have blocks of 256 threads");
+    auto run = [&](auto tiled, auto searched) {
+        auto kern = sparse ? searched : tiled;
+        kern<<<grid, 256, 0, s>>>(g.off, g.col, g.w, g.n, g.nnz, C, integral, acc);
         MG_LAUNCH_CHECK();
     };
-    if (g.wk == WK_UNIT) run(inner_weight_kernel<WK_UNIT>);
-    else if (g.wk == WK_F32) run(inner_weight_kernel<WK_F32>);
-    else if (g.wk == WK_U32) run(inner_weight_kernel<WK_U32>);
-    else run(inner_weight_kernel<WK_F64>);
+    if (g.wk == WK_UNIT) run(inner_weight_kernel<WK_UNIT>, inner_weight_sparse_kernel<WK_UNIT>);
+    else if (g.wk == WK_F32) run(inner_weight_kernel<WK_F32>, inner_weight_sparse_kernel<WK_F32>);
+    else if (g.wk == WK_U32) run(inner_weight_kernel<WK_U32>, inner_weight_sparse_kernel<WK_U32>);
+    else run(inner_weight_kernel<WK_F64>, inner_weight_sparse_kernel<WK_F64>);
 }
 
 double modularity_from_acc(const SweepAcc &a, double mass, int integral) {
