@@ -181,11 +181,16 @@ struct DBuf {
     T *ensure(size_t n) {
         if (n > cap) {
             // a large buffer that has to grow a little (the next graph is of
-            // about the same size) grows by a sixteenth more, memory permitting,
-            // so that not every new largest graph reallocates the workspace
+            // about the same size) grows by a sixteenth more, so that not every
+            // new largest graph reallocates the workspace -- while a sixteenth of
+            // the device's memory stays free, for buffers that have yet to grow
             const bool again = cap * sizeof(T) >= kSlackFrom && n < cap + cap / 4;
             release();
-            const size_t want = n < 16 ? 16 : n, roomy = again ? want + want / 16 : want;
+            const size_t want = n < 16 ? 16 : n;
+            size_t roomy = want, free_now = 0, total = 0;
+            if (again && cudaMemGetInfo(&free_now, &total) == cudaSuccess &&
+                free_now > total / 16 + (want + want / 16) * sizeof(T))
+                roomy = want + want / 16;
             if (alloc_fault_due()) throw Error(MG_ERR_OOM, "device allocation failed (injected by mg_test_fail_allocation)");
             size_t got = 0;
             if (pool && (p = (T *)pool->take(want * sizeof(T), got))) {

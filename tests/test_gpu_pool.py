@@ -103,3 +103,31 @@ def test_a_failed_call_leaves_no_copy_in_flight(mg):
         assert e.value.status == 3 and waited < 1e-3, waited
     assert c.graph_from_csr(9, *_ring(9)).info()["nnz"] == 36
     c.close()
+
+
+def test_a_workspace_grows_without_slack_on_a_full_device(mg):
+    """A workspace that grows for a slightly larger graph takes no more memory
+    than a new one when little of the device's memory is left."""
+    import torch
+
+    def used(sizes):
+        c = mg.Context(0)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for n in sizes:
+            g = c.generate_sbm(n, 64, 16.0, 0.8, seed=1)
+            g.louvain()
+            g.close()
+            c.trim()
+        after = torch.cuda.mem_get_info()[0]
+        c.close()
+        return before - after
+
+    used([100000])
+    free, total = torch.cuda.mem_get_info()
+    hold = torch.empty(free - (total // 16 - (1 << 30)), dtype=torch.uint8, device="cuda")
+    try:
+        assert used([3000000, 3300000]) < used([3300000]) + (64 << 20)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
