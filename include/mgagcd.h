@@ -413,7 +413,8 @@ mg_status mg_batch_graph_info(const mg_batch *b, uint32_t g, uint32_t *n, uint64
 mg_status mg_batch_destroy(mg_batch *b);
 
 enum {
-    MG_BATCH_GRAPHS = 1 /* run each phase's iterations as one CUDA graph with a device-side loop */
+    MG_BATCH_GRAPHS = 1 /* run each phase's iterations as one CUDA graph with a device-side loop (phases that
+                           run in the resident kernel, which iterates by itself, take no notice) */
 };
 
 typedef struct {

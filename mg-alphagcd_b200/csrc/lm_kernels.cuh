@@ -1,6 +1,7 @@
 // lm_kernels.cuh -- the local-move sweep kernels and their launcher, shared by
 // the single-graph sweep (local_move.cu) and the batched sweep
-// (local_move_batch.cu).  Included by exactly those two translation units.
+// (local_move_batch.cu).  The resident kernels (resident_*.cu) and the step
+// between small levels (small_level.cu) use its device functions and helpers.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -407,8 +408,8 @@ __device__ __forceinline__ void group_argmax(G &best, uint32_t &dst, int up, G *
     }
 }
 
-// table bits for a vertex of degree d: 2*d slots rounded up to a power of
-// two, at least 32, at most the group's table (2^max_bits slots)
+// table bits for a vertex of degree d: the first power of two of at least 4*d
+// slots (32 up to degree 16), at most the group's table (2^max_bits slots)
 __device__ __forceinline__ int table_bits(uint32_t d, int max_bits) {
     const int want = d <= 16 ? 5 : 33 - __clz(2 * d - 1);
     return want < max_bits ? want : max_bits;

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kScanOneThreads) scan_one_kernel(const T *in, 
     if (d_total && threadIdx.x == kScanOneThreads - 1) *d_total = run;
 }
 
-// Tiles whose sums each block adds up itself (2 MB of reads over all blocks).
+// Tiles whose sums each block adds up itself (1 MB of reads over all blocks).
 constexpr size_t kScanSumTiles = 512;
 
 }  // namespace
