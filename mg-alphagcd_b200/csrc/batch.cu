@@ -628,13 +628,13 @@ int resident_team(const uint64_t *load, uint32_t graphs, int real, int sms) {
             sum += t;
             most = std::max(most, t);
         }
-        const double mean = sum * cs / sms, last = risk * most;
+        const double mean = sum / (sms / cs), last = risk * most;  // (whole clusters only)
         return std::max(last, mean) + part * std::min(last, mean);
     };
     auto classes = [&](double rate, double launches) { return total / (rate / kNumSMs * sms) + launches; };
     double best = classes(46e3, 120);
     int ctas = 0;
-    for (int cs = 1; cs <= 8; cs *= 2) {
+    for (int cs = 1; cs <= 8 && cs <= sms; cs *= 2) {
         const double est = team(cs, 440, 1, 0.35);
         if (est < best) {
             best = est;
