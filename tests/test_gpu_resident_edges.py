@@ -96,3 +96,23 @@ def test_class_kernels_in_every_precision(O, ctx, name, precision, version):
     if precision == "fp64":
         _same(a, ref)
     dg.close()
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_batch_launch_modes_of_the_class_kernels(O, mg, ctx, graphs):
+    """Batches of small graphs run resident by default, whatever launch mode is
+    asked for; with the shapes fixed, both modes of the class kernels run."""
+    from test_gpu_batch import _check_graph, _mixed_graphs, _pack
+
+    gs = _mixed_graphs(O)
+    b = _pack(ctx, gs)
+    ctx.tune_mode(mg.TUNE_OFF)
+    try:
+        res = b.run(graphs=graphs)
+    finally:
+        ctx.tune_mode(mg.TUNE_ON)
+    assert res["kernel_launches"] > b.run()["kernel_launches"]
+    for i, g in enumerate(gs):
+        if g.nnz:
+            _check_graph(res, i, O.louvain(g))
+    b.close()
